@@ -79,11 +79,13 @@ namespace zeus {
       }
     }
 
+    // (unrolled whole where a thread holds x in registers: a partly unrolled
+    // loop indexes x dynamically, which puts it in local memory)
     __host__ __device__ double
     value(const double* x) const
     {
       double sum = 0.0;
-#pragma unroll 4
+#pragma unroll(D <= 16 ? 16 : 4)
       for (std::size_t i = 0; i + 1 < D; ++i) {
         const double t1 = 1.0 - x[i];
         const double t2 = fma(-x[i], x[i], x[i + 1]);
@@ -113,20 +115,43 @@ namespace zeus {
       return (acc[0] + acc[1]) + (acc[2] + acc[3]);
     }
 
-    // d/dx_i: -2(1-x_i) - 400 x_i (x_{i+1}-x_i^2) + 200 (x_i - x_{i-1}^2)
+    // d/dx_i: -2(1-x_i) - 400 x_i (x_{i+1}-x_i^2) + 200 (x_i - x_{i-1}^2).
+    // Up to D = 16 the loop is unrolled whole (x and g then stay in a
+    // thread's registers) and its roundings are written out: those of the
+    // loop that takes (D - 1) % 4 terms, then four at a time, where the
+    // previous term's 200 t2 is fused into the next entry inside a group of
+    // four and rounded on its own where a group begins.
     __host__ __device__ double
     adjoint(const double* x, double* g) const
     {
-      double sum = 0.0, carry = 0.0;
+      double sum = 0.0;
+      if constexpr (D <= 16) {
+        constexpr int first = ((int)D - 1) % 4;
+        double tp = 0.0; // the previous term's t2
+#pragma unroll
+        for (int i = 0; i + 1 < (int)D; ++i) {
+          const double t1 = 1.0 - x[i];
+          const double t2 = fma(-x[i], x[i], x[i + 1]);
+          sum = fma(100.0 * t2, t2, fma(t1, t1, sum));
+          const double lead = i == 0                ? -2.0 * t1
+                              : (i - first) % 4 == 0 ? fma(-2.0, t1, 200.0 * tp)
+                                                     : fma(200.0, tp, -2.0 * t1);
+          g[i] = fma(-(400.0 * x[i]), t2, lead);
+          tp = t2;
+        }
+        g[D - 1] = 200.0 * tp;
+      } else {
+        double carry = 0.0;
 #pragma unroll 4
-      for (std::size_t i = 0; i + 1 < D; ++i) {
-        const double t1 = 1.0 - x[i];
-        const double t2 = fma(-x[i], x[i], x[i + 1]);
-        sum = fma(100.0 * t2, t2, fma(t1, t1, sum));
-        g[i] = carry - 2.0 * t1 - 400.0 * x[i] * t2;
-        carry = 200.0 * t2;
+        for (std::size_t i = 0; i + 1 < D; ++i) {
+          const double t1 = 1.0 - x[i];
+          const double t2 = fma(-x[i], x[i], x[i + 1]);
+          sum = fma(100.0 * t2, t2, fma(t1, t1, sum));
+          g[i] = carry - 2.0 * t1 - 400.0 * x[i] * t2;
+          carry = 200.0 * t2;
+        }
+        g[D - 1] = carry;
       }
-      g[D - 1] = carry;
       return sum;
     }
 
