@@ -128,6 +128,18 @@ namespace zb {
     { f.value_line(xp, a) } -> std::convertible_to<double>;
   };
 
+  // Objectives whose cooperative value evaluates several line-search trials
+  // in one sweep over their data (value_trials).
+  template <class F, int TS>
+  constexpr bool
+  has_value_trials()
+  {
+    if constexpr (requires { F::kTrialsAtOnce; })
+      return TS == 32; // a lane for every trial
+    else
+      return false;
+  }
+
   // One run on a tile: `buf` is the tile's tile_smem_doubles<D, TS>()
   // doubles of shared memory (16-byte aligned); start x0[D]; results to
   // slot `run` of `out`.
@@ -149,6 +161,7 @@ namespace zb {
     constexpr int R = (D + TS - 1) / TS;
     constexpr bool kLine = HasValueLine<F>;
     constexpr bool kCoopFirst = !kLine || D > 8;
+    constexpr bool kSweep = !kLine && has_value_trials<F, TS>();
     const int lane = (int)tile.thread_rank();
     double* xs = buf;
     double* gs = xs + D;
@@ -192,6 +205,7 @@ namespace zb {
       stop = v[1] != 0.0;
     }
     bool pend = false;
+    bool stalled = false; // the last search ended without a passing trial
     long long n_eval = 1, n_grad = 1;
     int status = kUnset, iter, executed = -1;
     double fout = best, gout = 0.0;
@@ -210,7 +224,10 @@ namespace zb {
       // else alpha = 2^-20 (utils.cuh:376-412)
       int found = -1;
       double fnew = 0.0;
-      if constexpr (kCoopFirst) {
+      // (after a search in which no trial passed, a sweep of several trials
+      // starts at trial 0: the next search will most likely fail too)
+      int k0 = kCoopFirst && !(kSweep && stalled) ? 1 : 0;
+      if (k0 == 1) {
         grp.sync(); // earlier readers of xs are done
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -228,7 +245,6 @@ namespace zb {
         }
       }
       if (found < 0) {
-        constexpr int k0 = kCoopFirst ? 1 : 0;
         if constexpr (kLine) {
           grp.sync(); // earlier readers of xp are done
 #pragma unroll
@@ -257,6 +273,39 @@ namespace zb {
               fnew = tile.shfl(fk, wl);
             }
           }
+        } else if constexpr (kSweep) {
+          // kTrialsAtOnce trials to a sweep over the objective's data: a run
+          // whose trials all fail (one that iterates to MAX_ITER) waits for
+          // three sweeps and reductions instead of 20
+          constexpr int NK = F::kTrialsAtOnce;
+          grp.sync(); // earlier readers of xp are done
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const int i = lane + r * TS;
+            if (i < D)
+              *reinterpret_cast<double2*>(xp + 2 * i) = make_double2(x[r], p[r]);
+          }
+          grp.sync();
+          if (k0 == 0 && lane == 0)
+            stop_now = load_stop(ctl);
+          const double logs = f.trial_log(grp, reinterpret_cast<const double2*>(xp));
+          for (int base = k0; found < 0; base += NK) {
+            double fv[NK];
+            f.template value_trials<NK>(grp, reinterpret_cast<const double2*>(xp), logs, base,
+                                        fv);
+#pragma unroll
+            for (int q = NK - 1; q >= 0; --q) {
+              const int k = base + q;
+              const double ak = pow2neg(k);
+              if (k == kLineSearchTrials ||
+                  (k < kLineSearchTrials && fv[q] <= best + kArmijoC1 * ak * ddir &&
+                   fv[q] < best)) {
+                found = k;
+                fnew = fv[q];
+              }
+            }
+          }
+          stalled = found == kLineSearchTrials;
         } else {
           double a = pow2neg(k0);
           for (int k = k0; k <= kLineSearchTrials; ++k, a *= 0.5) {
