@@ -2,6 +2,7 @@
 // about D = 160 in a global-memory slice per block taken from the caller's
 // workspace).
 #include "zb_bfgs_coop.cuh"
+#include "zb_bfgs_quad.cuh"
 #include "zb_bfgs_rows.cuh"
 #include "zb_objective_visit.cuh"
 
@@ -25,6 +26,40 @@ namespace zb {
     {
       const int64_t cap = 2 * (int64_t)sm_count();
       return n < cap ? n : cap;
+    }
+
+    // The symmetric quadratic form with C in shared memory (zb_bfgs_quad.cuh):
+    // wherever a block's registers and shared memory hold H and C (D = 150), C
+    // is 16-byte aligned (the CTA layout splits a misaligned C's sums
+    // otherwise) and no cycle timers are asked for.
+    template <class F, int D>
+    constexpr bool
+    quad_built()
+    {
+      if constexpr (QuadraticForm<F> && D % 2 == 0 &&
+                    cta_block<D>() == kQuadSplitBlock)
+        return QuadShape<D>::fits;
+      else
+        return false;
+    }
+
+    template <class F, int D>
+    int
+    launch_quad(const F& f, const BfgsParams& prm, const double* starts, const RunOut& out,
+                Control* ctl, unsigned long long* queue, cudaStream_t st)
+    {
+      constexpr size_t smem = sizeof(double) * QuadShape<D>::doubles;
+      auto kern = bfgs_quad_kernel<F, D>;
+      int rc = cuda_fail(cudaFuncSetAttribute(
+                           kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                         "quadratic-form shared memory attribute");
+      if (rc || (rc = cuda_fail(cudaMemsetAsync(queue, 0, sizeof *queue, st),
+                                "quadratic-form run queue reset")))
+        return rc;
+      const int64_t cap = sm_count();
+      kern<<<(unsigned)(prm.n < cap ? prm.n : cap), QuadShape<D>::NT, smem, st>>>(
+        f, prm, starts, out, ctl, queue);
+      return cuda_fail(cudaGetLastError(), "quadratic-form BFGS launch");
     }
 
     template <class F, int D, bool Adj, bool kTimed>
@@ -60,6 +95,9 @@ namespace zb {
         return ZEUS_E_WORKSPACE;
       }
       auto* queue = static_cast<unsigned long long*>(ws);
+      if constexpr (quad_built<F, D>() && Adj && !kTimed)
+        if (f.symmetric && (reinterpret_cast<uintptr_t>(f.C) & 15u) == 0)
+          return launch_quad<F, D>(f, prm, starts, out, ctl, queue, st);
       double* hws = nullptr;
       if constexpr (cta_h_global(D, B)) {
         hws = reinterpret_cast<double*>(static_cast<char*>(ws) + kQueueBytes);
