@@ -17,6 +17,20 @@ namespace zb {
       const int64_t g = (int64_t)sm_count() * 4;
       return (int)(n < g ? n : g);
     }
+
+    // A warp per run up to D = 16; above, where a run's O(D^3) update is most
+    // of its time, only with more runs than two to an SM: below that a block's
+    // four warps on a run are the faster ones (Gaussian-32, 32 runs: 310 us
+    // against 350; 512 runs: 782 against 474).  The same line for the Poisson
+    // likelihood, whose evaluations take the same time in either form (100
+    // runs: 20.9 ms a block, 21.4 a warp).
+    bool
+    exact_warp_form(int kind, int dim, int64_t n)
+    {
+      if (dim > kExactWarpMaxDim)
+        return false;
+      return (dim <= 16 && kind != ZEUS_OBJ_POISSON_NLL) || n > 2 * (int64_t)sm_count();
+    }
   } // namespace
 
   bool
@@ -28,8 +42,8 @@ namespace zb {
   size_t
   exact_workspace_bytes(const Objective& o, int64_t n)
   {
-    if (n <= 0)
-      return 0;
+    if (n <= 0 || exact_warp_form(o.kind, o.dim, n))
+      return 0; // a warp per run keeps H and T in shared memory
     return sizeof(double) * 2 * (size_t)o.dim * o.dim * exact_grid(n);
   }
 
@@ -41,7 +55,7 @@ namespace zb {
     if (prm.n <= 0)
       return ZEUS_OK;
     const size_t need = exact_workspace_bytes(o, prm.n);
-    if (ws_bytes < need || !ws) {
+    if (need > 0 && (ws_bytes < need || !ws)) {
       set_error("exact BFGS needs %zu workspace bytes, got %zu", need,
                 ws_bytes);
       return ZEUS_E_WORKSPACE;
@@ -51,6 +65,23 @@ namespace zb {
     return visit_objective(o, [&](auto f) -> int {
       using F = decltype(f);
       constexpr int D = (int)F::arity;
+      if constexpr (D <= kExactWarpMaxDim) {
+        if (exact_warp_form(F::kind, D, prm.n)) {
+          constexpr int per = kExactWarpBlock / 32; // runs a block
+          constexpr size_t wsm = sizeof(double) * per * ExactWarpShape<D>::doubles;
+          auto kern = traj ? bfgs_exact_warp_kernel<F, D, true>
+                           : bfgs_exact_warp_kernel<F, D, false>;
+          if constexpr (wsm > 48 * 1024)
+            if (int rc = cuda_fail(cudaFuncSetAttribute(
+                                     kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)wsm),
+                                   "exact BFGS shared memory attribute"))
+              return rc;
+          kern<<<(unsigned)((prm.n + per - 1) / per), kExactWarpBlock, wsm, st>>>(
+            f, prm, starts, out, ctl);
+          return cuda_fail(cudaGetLastError(), "exact BFGS launch");
+        }
+      }
       const int grid = exact_grid(prm.n);
       const size_t smem = exact_smem_bytes<D>();
       double* scratch = static_cast<double*>(ws);
