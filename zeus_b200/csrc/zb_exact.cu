@@ -5,6 +5,7 @@
 #include "zb_objective_visit.cuh"
 #include "zb_pso.cuh"
 #include "zb_pso_dmma.cuh"
+#include "zb_pso_swarm.cuh"
 
 namespace zb {
 
@@ -114,6 +115,84 @@ namespace zb {
     return b;
   }
 
+  namespace {
+    // Particles a block of the one-launch PSO takes and whether C goes to
+    // shared memory; per = 0: the swarm does not fit, and each iteration is a
+    // launch.  A block holds at least kSwarmElems (particle, coordinate)
+    // elements, so a small swarm is one block and needs no meeting, and a
+    // large one is spread over the SMs.
+    constexpr int64_t kSwarmElems = 1024;
+
+    template <class F, int D>
+    int
+    swarm_per_block(int64_t n, int iters, bool* matrix)
+    {
+      constexpr int64_t limit = 227 * 1024 / sizeof(double) - 160; // static arrays
+      *matrix = false;
+      if (iters < 1)
+        return 0; // nothing to meet for
+      const int64_t sms = sm_count() < kSwarmMaxBlocks ? sm_count() : kSwarmMaxBlocks;
+      int64_t per = (n + sms - 1) / sms;
+      const int64_t least = (kSwarmElems + D - 1) / D;
+      per = per > least ? per : least;
+      per = per < n ? per : n;
+      if constexpr (swarm_dmma<F, D>()) {
+        per = (per + kPsoDmmaParticles - 1) / kPsoDmmaParticles * kPsoDmmaParticles;
+        // eight particles and C to a block: with C in L2 the blocks of a
+        // launch an iteration hide its latency better, several to an SM
+        // (4096 particles at D = 150: 213 us that way, 234 this way)
+        if (per > kPsoDmmaParticles || (int64_t)swarm_doubles<F, D>(per, true) > limit)
+          return 0;
+        *matrix = true;
+      } else if constexpr (F::kind == ZEUS_OBJ_GAUSSIAN) {
+        *matrix = true; // D x D is small
+      }
+      if (per > swarm_threads<F, D>() || (int64_t)swarm_doubles<F, D>(per, *matrix) > limit)
+        return 0;
+      return (int)per;
+    }
+
+    template <class F, int D, bool Matrix>
+    int
+    launch_swarm(const F& f, const SwarmArgs& a, unsigned blocks, cudaStream_t st)
+    {
+      auto kern = pso_swarm_kernel<F, D, Matrix>;
+      const size_t smem = sizeof(double) * swarm_doubles<F, D>(a.per_block, Matrix);
+      int rc = ZEUS_OK;
+      if (smem > 40 * 1024 &&
+          (rc = cuda_fail(cudaFuncSetAttribute(
+                            kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                          "PSO shared memory attribute")))
+        return rc;
+      if (blocks > 1 &&
+          (rc = cuda_fail(cudaMemsetAsync(a.slots, 0,
+                                          sizeof(unsigned long long) * 8 * blocks, st),
+                          "PSO slot reset")))
+        return rc;
+      cudaLaunchAttribute attr{};
+      attr.id = cudaLaunchAttributeCooperative;
+      attr.val.cooperative = 1;
+      cudaLaunchConfig_t lc{};
+      lc.gridDim = dim3(blocks);
+      lc.blockDim = dim3(swarm_threads<F, D>());
+      lc.dynamicSmemBytes = smem;
+      lc.stream = st;
+      lc.attrs = &attr;
+      lc.numAttrs = blocks > 1 ? 1 : 0;
+      return cuda_fail(cudaLaunchKernelEx(&lc, kern, f, a), "PSO launch");
+    }
+  } // namespace
+
+  bool
+  pso_one_launch(const Objective& o, int64_t n, int iters)
+  {
+    return visit_objective(o, [&](auto f) -> int {
+             using F = decltype(f);
+             bool m;
+             return swarm_per_block<F, (int)F::arity>(n, iters, &m) > 0 ? 1 : 0;
+           }) == 1;
+  }
+
   int
   launch_pso(const Objective& o, uint64_t seed, int64_t n, double lower,
              double upper, int iters, double w, double c1, double c2,
@@ -144,6 +223,20 @@ namespace zb {
     return visit_objective(o, [&](auto f) -> int {
       using F = decltype(f);
       constexpr int D = (int)F::arity;
+      bool matrix = false;
+      if (const int per = swarm_per_block<F, D>(n, iters, &matrix)) {
+        // the slots lie in the workspace: 2 x (32 + 8 D) bytes a block of
+        // at least 1024 / D particles, within the positions' and velocities'
+        // 16 D n bytes
+        const unsigned nb = (unsigned)((n + per - 1) / per);
+        SwarmArgs a{n,     per, iters, lower, upper, w, c1, c2, seed, sobol, pbx, pbf, gbest,
+                    static_cast<unsigned long long*>(ws), nullptr};
+        a.slot_x = reinterpret_cast<double*>(a.slots + 8 * (size_t)nb);
+        if constexpr (F::kind == ZEUS_OBJ_GAUSSIAN) // (matrix)
+          return launch_swarm<F, D, true>(f, a, nb, st);
+        else
+          return launch_swarm<F, D, false>(f, a, nb, st);
+      }
       pso_reset_kernel<D><<<1, 256, 0, st>>>(wk);
       if constexpr (D >= kPsoCoopMinDim && D <= kPsoDmmaMaxDim &&
                     F::kind == ZEUS_OBJ_GAUSSIAN) {

@@ -38,6 +38,8 @@ namespace zb {
   // PSO (zb_exact.cu)
   bool pso_supported(int kind, int dim);
   size_t pso_workspace_bytes(int64_t n, int dim);
+  // whether launch_pso runs a swarm of n in one launch
+  bool pso_one_launch(const Objective& o, int64_t n, int iters);
   int launch_pso(const Objective& o, uint64_t seed, int64_t n, double lower,
                  double upper, int iters, double w, double c1, double c2,
                  double* pbx, double* pbf, double* gbest, void* ws,

@@ -44,6 +44,14 @@ namespace zb {
     out[3] = c3;
   }
 
+  // The uniform double of two Philox words.
+  __host__ __device__ inline double
+  uniform01_word(uint32_t hi, uint32_t lo)
+  {
+    const uint64_t bits = ((uint64_t)hi << 32) | lo;
+    return (double)(bits >> 11) * (1.0 / 9007199254740992.0);
+  }
+
   // Uniform double in [0, 1) with 53 random bits.  Counter = (run lo,
   // index/2, tag, run hi), key = seed; one Philox block serves two indices.
   __host__ __device__ inline double
@@ -53,8 +61,7 @@ namespace zb {
     philox4x32_10((uint32_t)run, index >> 1, tag, (uint32_t)(run >> 32),
                   (uint32_t)seed, (uint32_t)(seed >> 32), o);
     const int w = (int)(index & 1u) * 2;
-    const uint64_t bits = ((uint64_t)o[w] << 32) | o[w + 1];
-    return (double)(bits >> 11) * (1.0 / 9007199254740992.0);
+    return uniform01_word(o[w], o[w + 1]);
   }
 
 } // namespace zb

@@ -462,11 +462,11 @@ zeus_pso_device_prng(const zeus_problem* problem, uint64_t seed, int32_t prng,
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (st)
     cudaStreamIsCapturing(st, &cs);
-  if (!st || cs != cudaStreamCaptureStatusNone)
+  if (!st || cs != cudaStreamCaptureStatusNone || pso_one_launch(o, n, iters))
     return launch_pso(o, seed, n, lower, upper, iters, w, c1, c2, d_pbest_x,
                       d_pbest_f, d_gbest, d_workspace, workspace_bytes, st,
                       sobol);
-  // Capture init + iterations into one graph and launch it.
+  // A launch an iteration: capture them into one graph and launch it.
   rc = cuda_fail(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal),
                  "PSO capture begin");
   if (rc)
