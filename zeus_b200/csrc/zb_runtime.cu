@@ -150,19 +150,71 @@ namespace zb {
     bins[4 * i + 3] = ::lgamma(k + 1.0);
   }
 
-  __global__ void
-  starts_kernel(uint64_t seed, int64_t n, int dim, double lower, double upper,
-                double* __restrict__ out, const uint32_t* __restrict__ sobol)
+  // Start points.  An item is a pair of neighbouring coordinates of one run
+  // (Philox: one block of random words serves both) or one coordinate of
+  // kSobolRuns consecutive runs (Sobol': their points differ in the low bits
+  // of the run index alone, so the shift and the high bits' directions are
+  // found once).  `items` a run or chunk of runs; a thread walks the items
+  // with a fixed stride whose quotient and remainder by `items` are given, so
+  // it divides once.  What bounds it is the ten Philox rounds and the 64-bit
+  // conversions: 1 000 003 runs of 10 coordinates (80 MB) 58 -> 21 us against a
+  // thread, a Philox block and a 64-bit division an element; 100 000 Sobol'
+  // points of 150 coordinates 417 -> 69 us (B200).
+  inline constexpr int kSobolRuns = 8;
+  inline constexpr int kStartsBlock = 256;
+
+  template <bool Sobol, bool Pairs>
+  __global__ void __launch_bounds__(kStartsBlock)
+    starts_kernel(uint64_t seed, int64_t n, int dim, double lower, double upper,
+                  double* __restrict__ out, const uint32_t* __restrict__ sobol,
+                  int64_t total, int items, int64_t step_q, int step_r)
   {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n * dim)
-      return;
-    const int64_t i = e / dim;
-    const int d = (int)(e - i * dim);
+    const int64_t first = (int64_t)blockIdx.x * kStartsBlock + threadIdx.x;
+    const int64_t stride = (int64_t)gridDim.x * kStartsBlock;
+    const double width = upper - lower;
     // no contraction: the same bits as lower + (upper - lower) * u in C
-    out[e] = __dadd_rn(lower, __dmul_rn(upper - lower,
-                                        position01(sobol, seed, kTagStarts,
-                                                   (uint64_t)i, (uint32_t)d)));
+    const auto place = [&](double u) { return __dadd_rn(lower, __dmul_rn(width, u)); };
+    int64_t i = first / items;
+    int b = (int)(first - i * items);
+    for (int64_t e = first; e < total; e += stride) {
+      if constexpr (Sobol) {
+        const int64_t run = i * kSobolRuns;
+        const uint32_t* v = sobol + (size_t)b * kSobolBits;
+        uint32_t x = sobol_shift(seed, (uint32_t)b);
+        for (uint32_t m = (uint32_t)run; m; m &= m - 1u)
+          x ^= v[ctz32(m)];
+        const uint32_t v0 = v[0], v1 = v[1], v2 = v[2];
+        const int cnt = (int)(n - run < kSobolRuns ? n - run : kSobolRuns);
+        double* o = out + run * dim + b;
+#pragma unroll
+        for (int r = 0; r < kSobolRuns; ++r) {
+          const uint32_t y =
+            x ^ ((r & 1) ? v0 : 0u) ^ ((r & 2) ? v1 : 0u) ^ ((r & 4) ? v2 : 0u);
+          if (r < cnt)
+            o[(int64_t)r * dim] = place(((double)y + 0.5) * (1.0 / 4294967296.0));
+        }
+      } else {
+        uint32_t w[4];
+        philox4x32_10((uint32_t)i, (uint32_t)b, kTagStarts, (uint32_t)((uint64_t)i >> 32),
+                      (uint32_t)seed, (uint32_t)(seed >> 32), w);
+        const double u0 = place(uniform01_word(w[0], w[1]));
+        const double u1 = place(uniform01_word(w[2], w[3]));
+        double* o = out + i * dim + 2 * b;
+        if constexpr (Pairs) {
+          *reinterpret_cast<double2*>(o) = make_double2(u0, u1);
+        } else {
+          o[0] = u0;
+          if (2 * b + 1 < dim)
+            o[1] = u1;
+        }
+      }
+      i += step_q;
+      b += step_r;
+      if (b >= items) {
+        b -= items;
+        ++i;
+      }
+    }
   }
 
   __global__ void __launch_bounds__(256)
@@ -399,10 +451,19 @@ zeus_starts(uint64_t seed, int32_t prng, int64_t n, int32_t dim, double lower,
     return rc;
   if (n == 0)
     return ZEUS_OK;
-  const int64_t total = n * dim;
-  const unsigned grid = (unsigned)((total + 255) / 256);
-  starts_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(seed, n, dim, lower,
-                                                       upper, d_out, sobol);
+  const int items = sobol ? dim : (dim + 1) / 2;
+  const int64_t total = (sobol ? (n + kSobolRuns - 1) / kSobolRuns : n) * items;
+  const int64_t most = (int64_t)sm_count() * 8;
+  const int64_t need = (total + kStartsBlock - 1) / kStartsBlock;
+  const unsigned grid = (unsigned)(need < most ? need : most);
+  const int64_t stride = (int64_t)grid * kStartsBlock;
+  // pairs are stored as one where every pair is 16-byte aligned
+  const bool pairs = dim % 2 == 0 && (reinterpret_cast<uintptr_t>(d_out) & 15u) == 0;
+  auto kern = sobol ? starts_kernel<true, false>
+                    : pairs ? starts_kernel<false, true> : starts_kernel<false, false>;
+  kern<<<grid, kStartsBlock, 0, (cudaStream_t)stream>>>(
+    seed, n, dim, lower, upper, d_out, sobol, total, items, stride / items,
+    (int)(stride % items));
   return cuda_fail(cudaGetLastError(), "starts launch");
 }
 
