@@ -1,6 +1,7 @@
 // Final reduction over runs: argmin of fval plus the status census, one
-// kernel (the reference runs a CUB ArgMin, copies every Result<D> to the
-// host and counts there: bfgs_common.cuh:280-319, util.hpp:151-200).
+// kernel (census_kernel, zb_runtime.cu; the reference runs a CUB ArgMin, copies
+// every Result<D> to the host and counts there: bfgs_common.cuh:280-319,
+// util.hpp:151-200).
 #pragma once
 
 #include "zb_common.cuh"
@@ -18,13 +19,6 @@ namespace zb {
   struct Census {
     int32_t actual, claimed, surrendered, stopped, best_idx, reserved;
   };
-
-  // One block of 1024 threads, grid-stride over the runs.
-  __global__ void __launch_bounds__(1024)
-    census_kernel(const double* __restrict__ fval,
-                  const int32_t* __restrict__ status,
-                  const double* __restrict__ x, int64_t n, int dim,
-                  KnownMin km, Census* out);
 
   // NLL per-bin constants {ln x, ln(1-x), k, lgamma(k+1)}.
   __global__ void nll_bins_kernel(const double* __restrict__ centres,

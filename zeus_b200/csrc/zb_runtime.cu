@@ -10,6 +10,8 @@
 #include <tuple>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "zb_internal.h"
 #include "zb_objective_visit.cuh"
 #include "zb_philox.cuh"
@@ -61,20 +63,39 @@ namespace zb {
     return v;
   }
 
+  // The census of a launch: one block, or a cluster of kCensusBlocks whose
+  // counts and minima meet in the first one's shared memory (no workspace, one
+  // launch).  A group of G lanes (the power of two at or above dim, at most a
+  // warp) takes a run's coordinates, kCensusRuns runs in flight a group; its
+  // sum of squares is the xor tree of a warp whose lanes past G add zeros,
+  // for any G.  One block with a warp a run waited for one load after another:
+  // 16384 runs of 10 coordinates 255 -> 24 us, 131072 of 4 2.0 ms -> 50 us,
+  // 1 000 000 of 10 15.9 -> 1.2 ms (B200); up to 2048 runs a cluster's launch
+  // costs what it saves.
+  inline constexpr int kCensusBlocks = 8;
+  inline constexpr int kCensusRuns = 4;
+  inline constexpr int64_t kCensusOneBlock = 2048; // runs up to which one block does
+
+  template <int G>
   __global__ void __launch_bounds__(1024)
-    census_kernel(const double* __restrict__ fval,
-                  const int32_t* __restrict__ status,
+    census_kernel(const double* __restrict__ fval, const int32_t* __restrict__ status,
                   const double* __restrict__ x, int64_t n, int dim,
-                  KnownMin km, Census* out)
+                  const __grid_constant__ KnownMin km, Census* out)
   {
     __shared__ int cnt[4];
+    __shared__ unsigned long long best_key;
+    __shared__ int best_idx;
+    const int lane = threadIdx.x & 31;
     if (threadIdx.x < 4)
       cnt[threadIdx.x] = 0;
     __syncthreads();
     unsigned long long key = ~0ull;
     int idx = 0x7fffffff;
     int actual = 0, claimed = 0, stopped = 0, surr = 0;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t threads = (int64_t)gridDim.x * blockDim.x;
+#pragma unroll 4
+    for (int64_t i = tid; i < n; i += threads) {
       const unsigned long long k = order_key(fval[i]);
       if (k < key || (k == key && (int)i < idx)) {
         key = k;
@@ -89,49 +110,78 @@ namespace zb {
         ++surr;
     }
     if (x) {
-      // converged runs within 0.5 of the known minimum: a warp per run, its
-      // lanes over the coordinates (coalesced rows of x), four runs in flight
-      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-      const int nw = blockDim.x >> 5;
-      constexpr int R = 4;
-      for (int64_t i0 = (int64_t)warp * R; i0 < n; i0 += (int64_t)nw * R) {
-        double ss[R];
-        bool conv[R];
+      // converged runs within 0.5 of the known minimum
+      const int64_t groups = threads / G;
+      const int m = threadIdx.x % G;
+      for (int64_t i0 = tid / G; i0 - lane / G < n; i0 += groups * kCensusRuns) {
+        double ss[kCensusRuns];
+        bool conv[kCensusRuns];
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int64_t i = i0 + r;
+        for (int r = 0; r < kCensusRuns; ++r) {
+          const int64_t i = i0 + r * groups;
           conv[r] = i < n && status[i] == kConverged;
+        }
+#pragma unroll
+        for (int r = 0; r < kCensusRuns; ++r) {
+          const int64_t i = i0 + r * groups;
           ss[r] = 0.0;
           if (conv[r])
-            for (int d = lane; d < dim; d += 32) {
+            for (int d = m; d < dim; d += G) {
               const double df = x[i * dim + d] - (km.has ? km.x[d] : 0.0);
               ss[r] = fma(df, df, ss[r]);
             }
         }
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
+        for (int r = 0; r < kCensusRuns; ++r) {
 #pragma unroll
-          for (int m = 16; m > 0; m >>= 1)
-            ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], m);
-          if (lane == 0 && conv[r] && sqrt(ss[r]) < 0.5)
+          for (int o = G / 2; o > 0; o >>= 1)
+            ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], o);
+          if (m == 0 && conv[r] && sqrt(ss[r]) < 0.5)
             ++actual;
         }
       }
     }
-    atomicAdd(&cnt[0], actual);
-    atomicAdd(&cnt[1], claimed);
-    atomicAdd(&cnt[2], surr);
-    atomicAdd(&cnt[3], stopped);
+    const int sums[4] = {__reduce_add_sync(0xffffffffu, actual),
+                         __reduce_add_sync(0xffffffffu, claimed),
+                         __reduce_add_sync(0xffffffffu, surr),
+                         __reduce_add_sync(0xffffffffu, stopped)};
+    if (lane == 0)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (sums[q])
+          atomicAdd(&cnt[q], sums[q]);
     block_argmin(key, idx);
-    __syncthreads();
     if (threadIdx.x == 0) {
-      out->actual = cnt[0];
-      out->claimed = cnt[1];
-      out->surrendered = cnt[2];
-      out->stopped = cnt[3];
+      best_key = key;
+      best_idx = idx;
+    }
+    __syncthreads();
+    const cg::cluster_group cluster = cg::this_cluster();
+    const int nb = (int)gridDim.x; // the grid is one cluster
+    if (nb > 1)
+      cluster.sync();
+    if (cluster.block_rank() == 0 && threadIdx.x == 0) {
+      int total[4] = {cnt[0], cnt[1], cnt[2], cnt[3]};
+      for (int b = 1; b < nb; ++b) {
+        const int* c = cluster.map_shared_rank(cnt, b);
+        for (int q = 0; q < 4; ++q)
+          total[q] += c[q];
+        const unsigned long long k = *cluster.map_shared_rank(&best_key, b);
+        const int ki = *cluster.map_shared_rank(&best_idx, b);
+        if (k < key || (k == key && ki < idx)) {
+          key = k;
+          idx = ki;
+        }
+      }
+      out->actual = total[0];
+      out->claimed = total[1];
+      out->surrendered = total[2];
+      out->stopped = total[3];
       out->best_idx = (n > 0 && idx != 0x7fffffff) ? idx : -1;
       out->reserved = 0;
     }
+    if (nb > 1)
+      cluster.sync(); // the first block has read the others' shared memory
   }
 
   __global__ void
@@ -718,9 +768,24 @@ zeus_census_device(const double* d_fval, const int32_t* d_status,
   km.has = known_min ? 1 : 0;
   for (int d = 0; d < kMaxKnownDim; ++d)
     km.x[d] = (known_min && d < dim) ? known_min[d] : 0.0;
-  census_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(
-    d_fval, d_status, d_x, n, dim, km, reinterpret_cast<Census*>(d_census));
-  return cuda_fail(cudaGetLastError(), "census launch");
+  auto kern = dim <= 2    ? census_kernel<2>
+              : dim <= 4  ? census_kernel<4>
+              : dim <= 8  ? census_kernel<8>
+              : dim <= 16 ? census_kernel<16>
+                          : census_kernel<32>;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = n > kCensusOneBlock ? kCensusBlocks : 1;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = dim3(attr.val.clusterDim.x);
+  lc.blockDim = dim3(1024);
+  lc.stream = (cudaStream_t)stream;
+  lc.attrs = &attr;
+  lc.numAttrs = 1;
+  return cuda_fail(cudaLaunchKernelEx(&lc, kern, d_fval, d_status, d_x, n, (int)dim, km,
+                                      reinterpret_cast<Census*>(d_census)),
+                   "census launch");
 }
 
 int
