@@ -150,7 +150,7 @@ namespace zb {
   // goes lane-per-trial).  Then one pass over the H rows in registers
   // applies the previous iteration's deferred update H += s w^T + w s^T and
   // forms u = H y and h = H g_next together, and one butterfly reduction of
-  // {s.y, y.u, u.g, s.g, g.h, g.g, stop} gives every scalar:
+  // {s.y, y.u, u.g, s.g, g.h, g.g} gives every scalar:
   //   p+ = -(h + s (w.g) + w (s.g)),  g.p+ = -(g.h + 2 (s.g)(w.g)).
   template <class F, int D, int TS, bool Adjoint, bool kTimed = false>
   __device__ __forceinline__ void
@@ -190,9 +190,8 @@ namespace zb {
     grp.sync();
     tm.stop_grad();
     double ddir;
-    bool stop;
     {
-      double v[2] = {0.0, lane == 0 ? (double)load_stop(ctl) : 0.0};
+      double v[1] = {0.0};
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const int i = lane + r * TS;
@@ -200,10 +199,13 @@ namespace zb {
         p[r] = -g[r];
         v[0] = fma(g[r], p[r], v[0]);
       }
-      grp.template sum<2>(v);
+      grp.template sum<1>(v);
       ddir = v[0];
-      stop = v[1] != 0.0;
     }
+    // the stop flag, tested every kStopEvery iterations on the value read at
+    // the previous test
+    int stop = load_stop(ctl);
+    const double tol_sq4 = 4.0 * prm.tol * prm.tol;
     bool pend = false;
     bool stalled = false; // the last search ended without a passing trial
     long long n_eval = 1, n_grad = 1;
@@ -211,23 +213,25 @@ namespace zb {
     double fout = best, gout = 0.0;
 
     for (iter = 0; iter < prm.max_iter; ++iter) {
-      if (stop) {
-        status = kStopped;
-        break;
+      if (iter % kStopEvery == 0) {
+        stop = grp.bcast(stop, 0);
+        if (stop) {
+          status = kStopped;
+          break;
+        }
+        stop = load_stop(ctl);
       }
-      // This iteration's read of the stop flag (consumed at the reduction)
-      // is issued after a sync and before a stretch of arithmetic: every
-      // sync waits for the thread's outstanding loads, so issued before one
-      // it would stall the tile for a global-memory round trip.
-      int stop_now = 0;
       // ---- line search: alpha_k = 2^-k, first k in 0..19 that passes,
       // else alpha = 2^-20 (utils.cuh:376-412)
       int found = -1;
       double fnew = 0.0;
       // (after a search in which no trial passed, a sweep of several trials
       // starts at trial 0: the next search will most likely fail too)
-      int k0 = kCoopFirst && !(kSweep && stalled) ? 1 : 0;
-      if (k0 == 1) {
+      constexpr int kFirst = kCoopFirst ? 1 : 0; // the first trial not on the whole tile
+      int k0 = kFirst;
+      if constexpr (kSweep)
+        k0 = stalled ? 0 : kFirst;
+      if (kCoopFirst && (!kSweep || k0 == 1)) {
         grp.sync(); // earlier readers of xs are done
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -236,8 +240,6 @@ namespace zb {
             xs[i] = fma(1.0, p[r], x[r]);
         }
         grp.sync();
-        if (lane == 0)
-          stop_now = load_stop(ctl);
         const double f0 = coop_value<F, D>(f, grp, xs);
         if (f0 <= best + kArmijoC1 * ddir && f0 < best) {
           found = 0;
@@ -254,9 +256,7 @@ namespace zb {
               *reinterpret_cast<double2*>(xp + 2 * i) = make_double2(x[r], p[r]);
           }
           grp.sync();
-          if (!kCoopFirst && lane == 0)
-            stop_now = load_stop(ctl);
-          for (int base = k0; found < 0; base += TS) {
+          for (int base = kFirst; found < 0; base += TS) {
             const int k = base + lane;
             double fk = 0.0;
             bool pass = false;
@@ -286,8 +286,6 @@ namespace zb {
               *reinterpret_cast<double2*>(xp + 2 * i) = make_double2(x[r], p[r]);
           }
           grp.sync();
-          if (k0 == 0 && lane == 0)
-            stop_now = load_stop(ctl);
           const double logs = f.trial_log(grp, reinterpret_cast<const double2*>(xp));
           for (int base = k0; found < 0; base += NK) {
             double fv[NK];
@@ -307,8 +305,8 @@ namespace zb {
           }
           stalled = found == kLineSearchTrials;
         } else {
-          double a = pow2neg(k0);
-          for (int k = k0; k <= kLineSearchTrials; ++k, a *= 0.5) {
+          double a = pow2neg(kFirst);
+          for (int k = kFirst; k <= kLineSearchTrials; ++k, a *= 0.5) {
             grp.sync();
 #pragma unroll
             for (int r = 0; r < R; ++r) {
@@ -396,7 +394,7 @@ namespace zb {
           hh[r] = ha[r][0] + ha[r][1];
         }
       }
-      double v[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, (double)stop_now};
+      double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const int i = lane + r * TS;
@@ -409,7 +407,7 @@ namespace zb {
           v[5] = fma(gx[r], gx[r], v[5]);
         }
       }
-      grp.template sum<7>(v);
+      grp.template sum<6>(v);
       const bool skipped = fabs(v[0]) < kMinCurvature;
       const double sg = v[3], gh = v[4];
       double rho = 0.0, hb = 0.0, wg = 0.0;
@@ -436,7 +434,6 @@ namespace zb {
       tm.stop_update();
       pend = !skipped;
       ddir = skipped ? -gh : -(gh + 2.0 * sg * wg);
-      stop = v[6] != 0.0;
       if (take) {
         best = fnew;
 #pragma unroll
@@ -445,19 +442,20 @@ namespace zb {
           g[r] = gn[r];
         }
       }
-      const double gnrm = sqrt(v[5]);
-      if (!isfinite(gnrm) || !isfinite(fnew)) {
+      // ||g|| = sqrt(g.g): taken only where it decides something (far
+      // above tol^2, g.g cannot pass the test)
+      if (!isfinite(v[5]) || !isfinite(fnew)) {
         status = kNonFinite;
         fout = fnew;
-        gout = gnrm;
+        gout = sqrt(v[5]);
         break;
       }
-      if (gnrm < prm.tol) {
+      if (v[5] <= tol_sq4 && sqrt(v[5]) < prm.tol) {
         if (lane == 0)
           note_converged(ctl, prm.required);
         status = kConverged;
         fout = best;
-        gout = gnrm;
+        gout = sqrt(v[5]);
         break;
       }
       if (!take && skipped && !(prm.flags & kFlagNoFixedPoint)) {

@@ -87,9 +87,6 @@ namespace zb {
       v[k] = __shfl_sync(0xffffffffu, a[0], RS::template owner<32>(k));
   }
 
-  // A block tests the stop flag every kQuadStopEvery iterations.
-  inline constexpr int kQuadStopEvery = 4;
-
   template <class F, int D>
   __global__ void __launch_bounds__(QuadShape<D>::NT, 1)
     bfgs_quad_kernel(F f, BfgsParams prm, const double* __restrict__ starts, RunOut out,
@@ -198,7 +195,7 @@ namespace zb {
         }
         __syncthreads(); // {x, p} and {s, w} are in place
         int stop_now = 0;
-        if (t == 0 && iter % kQuadStopEvery == 0)
+        if (t == 0 && iter % kStopEvery == 0)
           stop_now = load_stop(ctl);
         // ---- C x and C p, two chains of rows a segment
         if (works) {

@@ -106,13 +106,12 @@ namespace zb {
     int status = kUnset, iter, executed = -1;
     double fout = best, gout = 0.0;
     const double tol_sq4 = 4.0 * prm.tol * prm.tol;
-    // The stop flag: a warp's iteration can be shorter than the read's round
-    // trip to L2, so a warp tests it every kStopEvery iterations, on the
-    // value read at the previous test; a thread reads it one iteration ahead.
-    constexpr int kStopEvery = G > 1 ? 4 : 1;
+    // the stop flag: a warp tests it every kStopEvery iterations, on the value
+    // read at the previous test; a thread reads it one iteration ahead
+    constexpr int every = G > 1 ? kStopEvery : 1;
     int stop = load_stop(ctl);
     for (iter = 0; iter < prm.max_iter; ++iter) {
-      if (iter % kStopEvery == 0) {
+      if (iter % every == 0) {
         if constexpr (G > 1)
           stop = __shfl_sync(0xffffffffu, stop, 0);
         if (stop) {

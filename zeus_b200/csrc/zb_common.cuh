@@ -161,8 +161,12 @@ namespace zb {
     { f.adjoint(x, g) } -> std::convertible_to<double>;
   };
 
-  // Relaxed read of the stop flag, issued once per BFGS iteration like the
-  // reference's atomicAdd(&stopFlag, 0) (bfgs_common.cuh:127).
+  // Relaxed read of the stop flag (the reference's atomicAdd(&stopFlag, 0),
+  // once an iteration, bfgs_common.cuh:127).  Its round trip to L2 is as long as
+  // a short iteration, and a barrier waits for the loads its threads have in
+  // flight, so a group reads it every kStopEvery iterations and sees a raised
+  // flag that much later.
+  inline constexpr int kStopEvery = 4;
   __device__ __forceinline__ int
   load_stop(const Control* c)
   {
