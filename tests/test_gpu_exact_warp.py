@@ -47,3 +47,17 @@ def test_warp_form_equals_block_form(kind, dim):
     for name in ("x", "f", "g", "status"):
         np.testing.assert_array_equal(a.traj[name].cpu().numpy(),
                                       b.traj[name][..., :few].cpu().numpy(), err_msg=name)
+
+
+def test_workspace_of_many_runs_serves_few():
+    """A caller may size one workspace for its largest launch."""
+    import ctypes as C
+
+    import zeus_b200 as zb
+
+    cfg = zb.make_config(10, 1 << 30, 1e-8, "exact", "dual")
+    for obj in (zb.Rosenbrock(10), zb.Rosenbrock(32), zb.Ackley(30)):
+        p = obj.problem(None, None)
+        sizes = [zb.lib().zeus_bfgs_workspace_size(C.byref(p), C.byref(cfg), n)
+                 for n in (1, 40, 200, 1000, 20000)]
+        assert sizes == sorted(sizes) and sizes[0] > 0

@@ -43,8 +43,10 @@ namespace zb {
   size_t
   exact_workspace_bytes(const Objective& o, int64_t n)
   {
-    if (n <= 0 || exact_warp_form(o.kind, o.dim, n))
-      return 0; // a warp per run keeps H and T in shared memory
+    if (n <= 0)
+      return 0;
+    // what the block form takes, in either form's range: a workspace sized
+    // for many runs serves a later launch of few
     return sizeof(double) * 2 * (size_t)o.dim * o.dim * exact_grid(n);
   }
 
@@ -56,7 +58,7 @@ namespace zb {
     if (prm.n <= 0)
       return ZEUS_OK;
     const size_t need = exact_workspace_bytes(o, prm.n);
-    if (need > 0 && (ws_bytes < need || !ws)) {
+    if (ws_bytes < need || !ws) {
       set_error("exact BFGS needs %zu workspace bytes, got %zu", need,
                 ws_bytes);
       return ZEUS_E_WORKSPACE;
