@@ -1105,6 +1105,10 @@ zeus_autotune(const zeus_problem* problem, const zeus_bfgs_config* config,
     zeus_bfgs_config c = *config;
     c.layout = layout;
     c.tile = tile;
+    // the record also serves batches, whose kernel runs the thread layout a
+    // thread per run: that form is the one timed
+    if (layout == ZEUS_LAYOUT_THREAD && c.block <= 0)
+      c.block = 128;
     float ms_min = 3.4e38f;
     for (int rep = 0; rep < 2 && rc == ZEUS_OK; ++rep) { // warm-up + timed
       cudaMemsetAsync(ctl, 0, sizeof(int32_t) * 2, st);
