@@ -124,6 +124,9 @@ namespace zb {
     // elements, so a small swarm is one block and needs no meeting, and a
     // large one is spread over the SMs.
     constexpr int64_t kSwarmElems = 1024;
+    // the process may use fewer SMs than the device has (a shared device): the
+    // blocks cannot all be resident, and each iteration is a launch
+    constexpr int kSwarmNoRoom = 1;
 
     template <class F, int D>
     int
@@ -181,7 +184,12 @@ namespace zb {
       lc.stream = st;
       lc.attrs = &attr;
       lc.numAttrs = blocks > 1 ? 1 : 0;
-      return cuda_fail(cudaLaunchKernelEx(&lc, kern, f, a), "PSO launch");
+      const cudaError_t e = cudaLaunchKernelEx(&lc, kern, f, a);
+      if (e == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError();
+        return kSwarmNoRoom;
+      }
+      return cuda_fail(e, "PSO launch");
     }
   } // namespace
 
@@ -234,10 +242,11 @@ namespace zb {
         SwarmArgs a{n,     per, iters, lower, upper, w, c1, c2, seed, sobol, pbx, pbf, gbest,
                     static_cast<unsigned long long*>(ws), nullptr};
         a.slot_x = reinterpret_cast<double*>(a.slots + 8 * (size_t)nb);
-        if constexpr (F::kind == ZEUS_OBJ_GAUSSIAN) // (matrix)
-          return launch_swarm<F, D, true>(f, a, nb, st);
-        else
-          return launch_swarm<F, D, false>(f, a, nb, st);
+        // (the Gaussian's matrix is always in shared memory)
+        const int rc =
+          launch_swarm<F, D, F::kind == ZEUS_OBJ_GAUSSIAN>(f, a, nb, st);
+        if (rc != kSwarmNoRoom)
+          return rc;
       }
       pso_reset_kernel<D><<<1, 256, 0, st>>>(wk);
       if constexpr (D >= kPsoCoopMinDim && D <= kPsoDmmaMaxDim &&

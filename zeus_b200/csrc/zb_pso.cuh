@@ -1,5 +1,7 @@
 // PSO swarm seeding (the reference's pso.cuh:17-155), one particle per
-// thread, positions/velocities row-major [particle][dim] in HBM.
+// thread, positions/velocities row-major [particle][dim] in HBM: a launch an
+// iteration, for user objectives and for swarms past the one-launch kernel's
+// shared memory (zb_pso_swarm.cuh).
 //
 // Differences from the reference, by design:
 //  * random numbers come from the stateless Philox generator (zb_philox.cuh)
