@@ -108,11 +108,11 @@ def algorithmic_flops(jobs_counters) -> float:
 #    bytes written: the results stay in L2), scaled to the full batch by its
 #    runs (the bytes are the starts read and the results written, in
 #    proportion to the runs);
-#  * gaussian150: the CTA-layout BFGS kernel at full size (1.50 MB read: C,
-#    the starts and the first touch of the outputs).
+#  * gaussian150: the quadratic-form BFGS kernel at full size (C, the starts
+#    and the first touch of the outputs).
 MEASURED_TRAFFIC = {
     "mixed": (8 * (600064 + 1024), "1/8-size capture x 8, batch kernel"),
-    "gaussian150": (1503232, "full-size capture"),
+    "gaussian150": (1466000, "full-size capture"),
 }
 
 
@@ -427,7 +427,7 @@ def run_gpu(args, rank, world, local_rank):
                                        0.5, 1.2, 1.5, s["starts"].data_ptr(),
                                        p["pbf"].data_ptr(), p["gb"].data_ptr(),
                                        p["ws"].data_ptr(), p["wsz"], sh))
-            return 2 + j.pso_iter
+            return 1  # these swarms are one cooperative launch
         zb.check(L.zeus_starts_uniform(s["seed"], j.n, s["obj"].dim, j.lo, j.hi,
                                        s["starts"].data_ptr(), sh))
         return 1
