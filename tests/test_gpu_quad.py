@@ -46,3 +46,24 @@ def test_nonfinite_start_and_raised_stop_flag():
     r[0].launch(x0, reset_control=False)
     torch.cuda.synchronize()
     assert (r[0].status == 2).all() and (r[0].iter == 0).all()
+
+
+def test_matrix_that_is_not_16_byte_aligned():
+    """C at an odd double: the CTA layout's kernel, whose sums split otherwise."""
+    import torch
+
+    import zeus_b200 as zb
+
+    C = zb.gaussian_matrix(150)
+    dp = zb.device.DeviceProblem(zb.Gaussian(C))
+    buf = torch.zeros(1 + 150 * 150, dtype=torch.float64, device="cuda")
+    buf[1:] = dp.data.reshape(-1)
+    dp.data = buf[1:]
+    assert dp.data.data_ptr() % 16 == 8
+    x0 = torch.from_numpy(np.random.default_rng(2).uniform(-5, 5, (20, 150))).cuda()
+    r = [zb.bfgs_device(dp, x0, cycles=c) for c in (False, True)]
+    torch.cuda.synchronize()
+    assert (r[0].status == 1).all()
+    for name in ("fval", "status", "iter", "gnorm", "x", "counters"):
+        u, v = (getattr(q, name).cpu().numpy() for q in r)
+        np.testing.assert_array_equal(u, v, err_msg=name)
