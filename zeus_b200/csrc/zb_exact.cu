@@ -127,12 +127,14 @@ namespace zb {
     // the process may use fewer SMs than the device has (a shared device): the
     // blocks cannot all be resident, and each iteration is a launch
     constexpr int kSwarmNoRoom = 1;
+    // what a block's static arrays leave of an SM's shared memory
+    constexpr size_t kSwarmSmem = 227 * 1024 - 1280;
 
     template <class F, int D>
     int
     swarm_per_block(int64_t n, int iters, bool* matrix)
     {
-      constexpr int64_t limit = 227 * 1024 / sizeof(double) - 160; // static arrays
+      constexpr int64_t limit = kSwarmSmem / sizeof(double);
       *matrix = false;
       if (iters < 1)
         return 0; // nothing to meet for
@@ -164,9 +166,13 @@ namespace zb {
       auto kern = pso_swarm_kernel<F, D, Matrix>;
       const size_t smem = sizeof(double) * swarm_doubles<F, D>(a.per_block, Matrix);
       int rc = ZEUS_OK;
+      // the most a swarm takes, not what this one takes: the attribute is the
+      // kernel's, and a smaller swarm on another thread would lower it between
+      // this call's setting it and its launch
       if (smem > 40 * 1024 &&
           (rc = cuda_fail(cudaFuncSetAttribute(
-                            kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                            kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)kSwarmSmem),
                           "PSO shared memory attribute")))
         return rc;
       if (blocks > 1 &&
