@@ -204,6 +204,11 @@ int zeus_sobol_device_table(const uint32_t** d_table);
  * deterministic argmin, ties to the lowest index), all launched on `stream`
  * with no host round trip.  Outputs the per-particle best positions (the
  * BFGS starts, d_pbest_x[n*dim]) and values; d_gbest receives {f, x[dim]}.
+ * A swarm of several blocks in one launch has them wait for one another, with
+ * a limit of some two seconds.  If it runs out, the affected particles'
+ * positions and values and d_gbest[0] are NaN (f there is never NaN
+ * otherwise); the call has returned by then, so read d_gbest[0] where that
+ * matters.  zeus_optimize and zeus_batch_plan_run do, and return ZEUS_E_CUDA.
  * Workspace: zeus_pso_workspace_size() bytes of device memory. */
 size_t zeus_pso_workspace_size(int64_t n, int32_t dim);
 int zeus_pso_device(const zeus_problem* problem, uint64_t seed, int64_t n,
@@ -233,7 +238,8 @@ int zeus_pso_device_prng(const zeus_problem* problem, uint64_t seed,
  * address up (cudaGetSymbolAddress), so make that first call before any
  * stream capture.  All calls share the array and it keeps the last call's
  * contents; each call clears what must start at zero, but calls that
- * overlap on the GPU race on it: serialize them.  Outputs as for
+ * overlap on the GPU race on it, and may clear what the blocks of another
+ * wait for (see zeus_pso_device): serialize them.  Outputs as for
  * zeus_pso_device (Philox positions, as ZEUS_PRNG_PHILOX). */
 int zeus_pso_device_noalloc(const zeus_problem* problem, uint64_t seed,
                             int64_t n, double lower, double upper,

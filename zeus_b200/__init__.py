@@ -493,7 +493,7 @@ def _zeus_with_trajectories(f, lower, upper, N, MAX_ITER, PSO_ITER, required, to
     recording every iteration, the census, then the file."""
     import torch
 
-    from .device import bfgs_device, census_device, pso_device, starts
+    from .device import bfgs_device, census_device, check_swarm, pso_device, starts
 
     if not str(path).endswith(".tsv"):
         check(lib().zeus_write_trajectory_tsv(str(path).encode(), None, None, None, None,
@@ -501,8 +501,8 @@ def _zeus_with_trajectories(f, lower, upper, N, MAX_ITER, PSO_ITER, required, to
     if N == 0:
         return Result()
     if PSO_ITER >= 0:
-        x0, _, _ = pso_device(f, seed & 0xFFFFFFFFFFFFFFFF, N, lower, upper, PSO_ITER,
-                              prng=prng)
+        x0, _, gbest = pso_device(f, seed & 0xFFFFFFFFFFFFFFFF, N, lower, upper, PSO_ITER,
+                                  prng=prng)
     else:
         x0 = starts(seed & 0xFFFFFFFFFFFFFFFF, N, f.dim, lower, upper, prng=prng)
     r = bfgs_device(f, x0, max_iter=MAX_ITER, required=required, tol=tol,
@@ -510,6 +510,8 @@ def _zeus_with_trajectories(f, lower, upper, N, MAX_ITER, PSO_ITER, required, to
     cen = census_device(r.fval, r.status, r.x, f.dim,
                         np.ones(f.dim) if f.kind == OBJ_ROSENBROCK else None)
     torch.cuda.synchronize()
+    if PSO_ITER >= 0:
+        check_swarm(gbest)
     write_trajectory_tsv(path, r.traj)
     idx = int(cen["best_idx"])
     out = Result(idx=idx, status=int(r.status[idx]), fval=float(r.fval[idx]),

@@ -127,17 +127,24 @@ namespace zb {
     // the process may use fewer SMs than the device has (a shared device): the
     // blocks cannot all be resident, and each iteration is a launch
     constexpr int kSwarmNoRoom = 1;
+    // bins up to which a likelihood's swarm is one launch: the blocks that wait
+    // for the slowest evaluation (some 10 ms) are then far from their limit,
+    // and a launch an iteration is nothing beside longer ones
+    constexpr int kSwarmMaxBins = 8192;
     // what a block's static arrays leave of an SM's shared memory
     constexpr size_t kSwarmSmem = 227 * 1024 - 1280;
 
     template <class F, int D>
     int
-    swarm_per_block(int64_t n, int iters, bool* matrix)
+    swarm_per_block(const F& f, int64_t n, int iters, bool* matrix)
     {
       constexpr int64_t limit = kSwarmSmem / sizeof(double);
       *matrix = false;
       if (iters < 1)
         return 0; // nothing to meet for
+      if constexpr (F::kind == ZEUS_OBJ_POISSON_NLL)
+        if (f.nbins > kSwarmMaxBins)
+          return 0;
       const int64_t sms = sm_count() < kSwarmMaxBlocks ? sm_count() : kSwarmMaxBlocks;
       int64_t per = (n + sms - 1) / sms;
       const int64_t least = (kSwarmElems + D - 1) / D;
@@ -199,13 +206,20 @@ namespace zb {
     }
   } // namespace
 
+  extern "C" int*
+  zeus_internal_swarm_wait(void)
+  {
+    static thread_local int wait = kSwarmWait;
+    return &wait;
+  }
+
   bool
   pso_one_launch(const Objective& o, int64_t n, int iters)
   {
     return visit_objective(o, [&](auto f) -> int {
              using F = decltype(f);
              bool m;
-             return swarm_per_block<F, (int)F::arity>(n, iters, &m) > 0 ? 1 : 0;
+             return swarm_per_block<F, (int)F::arity>(f, n, iters, &m) > 0 ? 1 : 0;
            }) == 1;
   }
 
@@ -240,13 +254,14 @@ namespace zb {
       using F = decltype(f);
       constexpr int D = (int)F::arity;
       bool matrix = false;
-      if (const int per = swarm_per_block<F, D>(n, iters, &matrix)) {
+      if (const int per = swarm_per_block<F, D>(f, n, iters, &matrix)) {
         // the slots lie in the workspace: 2 x (32 + 8 D) bytes a block of
         // at least 1024 / D particles, within the positions' and velocities'
         // 16 D n bytes
         const unsigned nb = (unsigned)((n + per - 1) / per);
         SwarmArgs a{n,     per, iters, lower, upper, w, c1, c2, seed, sobol, pbx, pbf, gbest,
-                    static_cast<unsigned long long*>(ws), nullptr};
+                    static_cast<unsigned long long*>(ws), nullptr,
+                    *zeus_internal_swarm_wait()};
         a.slot_x = reinterpret_cast<double*>(a.slots + 8 * (size_t)nb);
         // (the Gaussian's matrix is always in shared memory)
         const int rc =

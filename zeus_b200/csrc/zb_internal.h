@@ -27,6 +27,9 @@ namespace zb {
   void set_error(const char* fmt, ...);
   int cuda_fail(cudaError_t e, const char* what);
   int sm_count();
+  // The error of a call whose swarm came back with NaN as gbest's value: a
+  // block's wait ran out (zb_pso_swarm.cuh).
+  int swarm_gave_up();
 
   // exact mode (zb_exact.cu)
   bool exact_supported(int kind, int dim);
@@ -38,6 +41,9 @@ namespace zb {
   // PSO (zb_exact.cu)
   bool pso_supported(int kind, int dim);
   size_t pso_workspace_bytes(int64_t n, int dim);
+  // The calling thread's limit on the one-launch PSO's wait (SwarmArgs::wait),
+  // for tests that make it run out.
+  extern "C" int* zeus_internal_swarm_wait(void);
   // whether launch_pso runs a swarm of n in one launch
   bool pso_one_launch(const Objective& o, int64_t n, int iters);
   int launch_pso(const Objective& o, uint64_t seed, int64_t n, double lower,

@@ -13,10 +13,11 @@
 //
 // The array is kNoAllocScratchBytes (8 MiB) of device memory that every GPU
 // which loads the library keeps until the process exits.  Every call shares
-// it: the last call's contents stay there, the kernels clear what must start
-// at zero (the launch counter and gBest) at the beginning of each call, and
-// two calls that overlap on the GPU (different streams, or other threads)
-// race on it and corrupt each other -- callers must serialize them.
+// it: the last call's contents stay there, each call clears what must start
+// at zero (the slots its blocks meet in, or the launch counter) at its
+// beginning, and two calls that overlap on the GPU (different streams, or other
+// threads) race on it, corrupt each other and may keep each other's blocks
+// waiting to their limit -- callers must serialize them.
 #include <mutex>
 
 #include "zb_internal.h"

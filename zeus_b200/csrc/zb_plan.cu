@@ -7,6 +7,7 @@
 // kernel, reduces every class (argmin + census) and gathers each class's
 // census and best run into one packed buffer that comes back with one
 // device-to-host copy and one stream synchronisation.
+#include <cmath>
 #include <cstring>
 #include <new>
 #include <vector>
@@ -19,8 +20,9 @@ namespace {
   constexpr int kMaxPlanClasses = 16;
 
   // per class in the packed result: census (3 doubles of 6 int32), then
-  // fval, gradient norm, status, iter, idx, then x[dim]
-  constexpr int kPackHead = 3 + 5;
+  // fval, gradient norm, status, iter, idx, gbest's value (0 without a swarm),
+  // then x[dim]
+  constexpr int kPackHead = 3 + 6;
 
   struct PlanClass {
     zeus_host_class shape; // as given at creation (host pointers unused)
@@ -51,6 +53,7 @@ namespace {
     const int32_t* status;
     const int32_t* iter;
     const double* x;
+    const double* gbest; // nullptr: no swarm
     int dim;
     int64_t pack_off;
   };
@@ -80,6 +83,7 @@ namespace {
       out[5] = b >= 0 ? (double)g.status[b] : -1.0;
       out[6] = b >= 0 ? (double)g.iter[b] : 0.0;
       out[7] = (double)b;
+      out[8] = g.gbest ? g.gbest[0] : 0.0;
     }
     for (int d = threadIdx.x; d < g.dim; d += blockDim.x)
       out[kPackHead + d] = b >= 0 ? g.x[(size_t)b * g.dim + d] : 0.0;
@@ -367,7 +371,9 @@ zeus_batch_plan_run(zeus_batch_plan* P, const zeus_host_class* classes,
                                  km.empty() ? nullptr : km.data(), k.d_cen, st)))
       return fail(rc);
     gt.e[i] = GatherEntry{k.d_cen, k.d_fval, k.d_gnorm, k.d_status, k.d_iter,
-                          k.d_x,   dim,      (int64_t)k.pack_off};
+                          k.d_x,
+                          !classes[i].starts && classes[i].pso_iter >= 0 ? k.d_gbest : nullptr,
+                          dim,     (int64_t)k.pack_off};
     maxdim = dim > maxdim ? dim : maxdim;
   }
   gather_kernel<<<nc, maxdim < 256 ? 128 : 256, 0, st>>>(gt, P->d_pack);
@@ -378,6 +384,9 @@ zeus_batch_plan_run(zeus_batch_plan* P, const zeus_host_class* classes,
                           "D2H results")) ||
       (rc = zb::cuda_fail(cudaStreamSynchronize(st), "batch run")))
     return fail(rc);
+  for (int i = 0; i < nc; ++i)
+    if (std::isnan(P->h_pack[P->cls[i].pack_off + 8]))
+      return fail(zb::swarm_gave_up());
   P->h2d_last = h2d;
   size_t xoff = 0;
   for (int i = 0; i < nc; ++i) {

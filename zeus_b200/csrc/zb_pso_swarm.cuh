@@ -19,8 +19,12 @@
 // where it beats gbest, position) in a slot tagged with the iteration, two
 // slots in turn, reads the others' until all have arrived and finds the swarm's
 // best by itself.
-// The launch is cooperative (every block resident); a block that waits past
-// kSwarmSpinLimit reads gives up, marks gbest's value NaN and returns.
+// The launch is cooperative (every block resident), so the wait is as long as
+// the slowest block's evaluation.  It has a limit all the same: a block that has
+// read the slots SwarmArgs::wait times gives up, fills its rows of pbx and pbf
+// and gbest's value with NaN and returns.  The blocks that wait for it do the
+// same, block 0 among them, so gbest's value is NaN (which no swarm's best is)
+// whenever a row is not the swarm's.
 #pragma once
 
 #include "zb_objectives.cuh"
@@ -29,7 +33,8 @@
 
 namespace zb {
 
-  inline constexpr int kSwarmSpinLimit = 1 << 24;
+  // Reads of the slots before a block gives up: about two seconds.
+  inline constexpr int kSwarmWait = 1 << 22;
   inline constexpr int kSwarmMaxBlocks = 160; // slots read by one block
   inline constexpr int kSwarmAhead = 4; // elements a thread moves ahead of gbest
 
@@ -47,6 +52,7 @@ namespace zb {
     // low words and the index, each below the iteration's tag
     unsigned long long* slots;
     double* slot_x; // [2][gridDim.x][D]
+    int wait;       // reads of the slots before a block gives up
   };
 
   // f as a sum of per-coordinate terms added in index order: term(x, i) for
@@ -475,9 +481,9 @@ namespace zb {
           kidx = 0x7fffffff;
           // every slot's words at once, until all are this iteration's
           constexpr int SL = kSwarmMaxBlocks / 32;
-          unsigned long long w[SL][3];
+          unsigned long long w[SL][3] = {};
           bool late = true;
-          for (int spins = 0; spins < kSwarmSpinLimit; ++spins) {
+          for (int reads = 0; reads < a.wait; ++reads) {
             bool all = true;
 #pragma unroll
             for (int k = 0; k < SL; ++k)
@@ -522,8 +528,13 @@ namespace zb {
       }
       __syncthreads();
       if (sh_late) {
+        const double nan = __longlong_as_double(0x7ff8000000000000ll);
         if (t == 0)
-          a.gbest[0] = __longlong_as_double(0x7ff8000000000000ll);
+          a.gbest[0] = nan;
+        for (int e = t; e < elems; e += NT)
+          a.pbx[i0 * D + e] = nan;
+        for (int p = t; p < cnt; p += NT)
+          a.pbf[i0 + p] = nan;
         return;
       }
       if (sh_win >= 0 && sh_f < gbf) {

@@ -43,6 +43,14 @@ namespace zb {
   }
 
   int
+  swarm_gave_up()
+  {
+    set_error("PSO: the swarm's blocks waited for one another past their limit; "
+              "the swarm is incomplete");
+    return ZEUS_E_CUDA;
+  }
+
+  int
   sm_count()
   {
     static std::mutex mu;
@@ -268,26 +276,28 @@ namespace zb {
   }
 
   // The best run (the census's best_idx) beside the census, so that a host
-  // call reads both with one copy: census (3 doubles) | fval | ||g|| |
-  // status, iter | x[dim].
-  inline constexpr int kBestHead = 3 + 3;
+  // call reads both with one copy: census (3 doubles) | gbest's value (0
+  // without a swarm) | fval | ||g|| | status, iter | x[dim].
+  inline constexpr int kBestHead = 3 + 4;
 
   __global__ void __launch_bounds__(128)
     best_run_kernel(const Census* __restrict__ cen, const double* __restrict__ fval,
                     const double* __restrict__ gnorm, const int32_t* __restrict__ status,
                     const int32_t* __restrict__ iter, const double* __restrict__ x, int dim,
-                    double* __restrict__ pack)
+                    const double* __restrict__ gbest, double* __restrict__ pack)
   {
     const int b = cen->best_idx;
-    if (threadIdx.x == 0)
+    if (threadIdx.x == 0) {
       *reinterpret_cast<Census*>(pack) = *cen;
+      pack[3] = gbest ? gbest[0] : 0.0;
+    }
     if (b < 0)
       return;
     if (threadIdx.x == 0) {
-      pack[3] = fval[b];
-      pack[4] = gnorm[b];
-      reinterpret_cast<int32_t*>(pack + 5)[0] = status[b];
-      reinterpret_cast<int32_t*>(pack + 5)[1] = iter[b];
+      pack[4] = fval[b];
+      pack[5] = gnorm[b];
+      reinterpret_cast<int32_t*>(pack + 6)[0] = status[b];
+      reinterpret_cast<int32_t*>(pack + 6)[1] = iter[b];
     }
     for (int d = threadIdx.x; d < dim; d += blockDim.x)
       pack[kBestHead + d] = x[(int64_t)b * dim + d];
@@ -950,7 +960,8 @@ zeus_optimize(const zeus_problem* hp, double lower, double upper, int64_t n,
                                km.empty() ? nullptr : km.data(), cen, st)))
     return fail(rc);
   best_run_kernel<<<1, 128, 0, st>>>(reinterpret_cast<const Census*>(cen), ro.fval, ro.gnorm,
-                                     ro.status, ro.iter, ro.x, dim, dbl(o_pack));
+                                     ro.status, ro.iter, ro.x, dim,
+                                     swarm ? dbl(o_gbest) : nullptr, dbl(o_pack));
   std::vector<double> pack(kBestHead + (size_t)dim);
   if ((rc = cuda_fail(cudaGetLastError(), "best run launch")) ||
       (rc = cuda_fail(cudaMemcpyAsync(pack.data(), dbl(o_pack), pack_bytes,
@@ -958,6 +969,8 @@ zeus_optimize(const zeus_problem* hp, double lower, double upper, int64_t n,
                       "D2H census and best run")) ||
       (rc = cuda_fail(cudaStreamSynchronize(st), "BFGS run")))
     return fail(rc);
+  if (std::isnan(pack[3]))
+    return fail(swarm_gave_up());
   zeus_census hc;
   std::memcpy(&hc, pack.data(), sizeof hc);
   if (census)
@@ -974,10 +987,10 @@ zeus_optimize(const zeus_problem* hp, double lower, double upper, int64_t n,
                         "D2H statuses")))
       return fail(rc);
     best->idx = hc.best_idx;
-    best->fval = pack[3];
-    best->gradient_norm = pack[4];
+    best->fval = pack[4];
+    best->gradient_norm = pack[5];
     int32_t si[2];
-    std::memcpy(si, &pack[5], sizeof si);
+    std::memcpy(si, &pack[6], sizeof si);
     best->status = si[0];
     best->iter = si[1];
     if (best_x)

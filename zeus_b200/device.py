@@ -11,8 +11,8 @@ from typing import Optional
 import numpy as np
 import torch
 
-from . import (BatchClass, BfgsConfig, Objective, RunOutputs, check, lib, make_config,
-               prng_code, LAYOUT_AUTO, PRNG_PHILOX, GRADPATH_QUADRATIC, _GRADS)
+from . import (BatchClass, BfgsConfig, Objective, RunOutputs, ZeusError, check, lib, make_config,
+               prng_code, E_CUDA, LAYOUT_AUTO, PRNG_PHILOX, GRADPATH_QUADRATIC, _GRADS)
 
 
 def _stream_handle(stream: Optional[torch.cuda.Stream]) -> int:
@@ -65,7 +65,8 @@ def pso_device(obj, seed: int, n: int, lower: float, upper: float, iters: int,
                w: float = 0.5, c1: float = 1.2, c2: float = 1.5, device="cuda",
                stream=None, prng=PRNG_PHILOX):
     """PSO seeding; returns (pbest_x (n, dim), pbest_f (n,), gbest (dim+1,)).
-    `prng` picks the initial positions' generator (Sobol' for SOBOL)."""
+    `prng` picks the initial positions' generator (Sobol' for SOBOL).  NaN as
+    gbest's value: the swarm is incomplete (check_swarm)."""
     dp = _as_problem(obj, device)
     dim = dp.obj.dim
     pbx = torch.empty((n, dim), dtype=torch.float64, device=device)
@@ -78,6 +79,14 @@ def pso_device(obj, seed: int, n: int, lower: float, upper: float, iters: int,
                                      upper, iters, w, c1, c2, _ptr(pbx), _ptr(pbf),
                                      _ptr(gb), _ptr(ws), wsz, _stream_handle(stream)))
     return pbx, pbf, gb
+
+
+def check_swarm(gbest: torch.Tensor) -> None:
+    """Raises where `gbest` of pso_device says that the swarm is incomplete
+    (NaN as its value); waits for it."""
+    if torch.isnan(gbest[0]).item():
+        raise ZeusError(E_CUDA, "PSO: the swarm's blocks waited for one another past their "
+                        "limit; the swarm is incomplete")
 
 
 class BfgsRun:

@@ -187,7 +187,7 @@ def sharded_optimize(obj, n: int, lower: float, upper: float, max_iter: int,
     its current CUDA device: starts of all n runs on every rank (PSO with
     pso_iter iterations when pso_iter >= 0, else uniform Philox starts), BFGS
     on this rank's shard, census and argmin merged across ranks."""
-    from .device import (DeviceProblem, bfgs_device, census_device, pso_device,
+    from .device import (DeviceProblem, bfgs_device, census_device, check_swarm, pso_device,
                          starts_uniform)
 
     dev = torch.device("cuda", torch.cuda.current_device())
@@ -196,7 +196,7 @@ def sharded_optimize(obj, n: int, lower: float, upper: float, max_iter: int,
 
     def local(start: int, count: int) -> LocalCensus:
         if pso_iter >= 0:
-            allst, _, _ = pso_device(dp, seed, n, lower, upper, pso_iter, device=dev)
+            allst, _, gbest = pso_device(dp, seed, n, lower, upper, pso_iter, device=dev)
         else:
             allst = starts_uniform(seed, n, dim, lower, upper, device=dev)
         if count == 0:
@@ -207,6 +207,8 @@ def sharded_optimize(obj, n: int, lower: float, upper: float, max_iter: int,
         r = bfgs_device(dp, st, max_iter=max_iter, required=req, tol=tolerance,
                         gradient=gradient, layout=layout)
         c = census_device(r.fval, r.status, r.x, dim, known_min)
+        if pso_iter >= 0:
+            check_swarm(gbest)
         b = int(c["best_idx"])
         out = LocalCensus(c["actual"], c["claimed"], c["surrendered"], c["stopped"], b)
         if b >= 0:
