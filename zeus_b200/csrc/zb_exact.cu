@@ -124,8 +124,8 @@ namespace zb {
     // elements, so a small swarm is one block and needs no meeting, and a
     // large one is spread over the SMs.
     constexpr int64_t kSwarmElems = 1024;
-    // the process may use fewer SMs than the device has (a shared device): the
-    // blocks cannot all be resident, and each iteration is a launch
+    // the driver has no room for all blocks at once after all: each iteration
+    // is a launch
     constexpr int kSwarmNoRoom = 1;
     // bins up to which a likelihood's swarm is one launch: the blocks that wait
     // for the slowest evaluation (some 10 ms) are then far from their limit,
@@ -136,7 +136,7 @@ namespace zb {
 
     template <class F, int D>
     int
-    swarm_per_block(const F& f, int64_t n, int iters, bool* matrix)
+    swarm_per_block(const F& f, int64_t n, int iters, cudaStream_t st, bool* matrix)
     {
       constexpr int64_t limit = kSwarmSmem / sizeof(double);
       *matrix = false;
@@ -145,9 +145,12 @@ namespace zb {
       if constexpr (F::kind == ZEUS_OBJ_POISSON_NLL)
         if (f.nbins > kSwarmMaxBins)
           return 0;
-      const int64_t sms = sm_count() < kSwarmMaxBlocks ? sm_count() : kSwarmMaxBlocks;
-      int64_t per = (n + sms - 1) / sms;
       const int64_t least = (kSwarmElems + D - 1) / D;
+      // the blocks wait for one another, so there are no more than the stream
+      // has SMs (a graph that records the launch has no other check)
+      const int64_t has = n > least ? stream_sm_count(st) : 1;
+      const int64_t sms = has < kSwarmMaxBlocks ? has : kSwarmMaxBlocks;
+      int64_t per = (n + sms - 1) / sms;
       per = per > least ? per : least;
       per = per < n ? per : n;
       if constexpr (swarm_dmma<F, D>()) {
@@ -214,12 +217,12 @@ namespace zb {
   }
 
   bool
-  pso_one_launch(const Objective& o, int64_t n, int iters)
+  pso_one_launch(const Objective& o, int64_t n, int iters, cudaStream_t st)
   {
     return visit_objective(o, [&](auto f) -> int {
              using F = decltype(f);
              bool m;
-             return swarm_per_block<F, (int)F::arity>(f, n, iters, &m) > 0 ? 1 : 0;
+             return swarm_per_block<F, (int)F::arity>(f, n, iters, st, &m) > 0 ? 1 : 0;
            }) == 1;
   }
 
@@ -254,7 +257,7 @@ namespace zb {
       using F = decltype(f);
       constexpr int D = (int)F::arity;
       bool matrix = false;
-      if (const int per = swarm_per_block<F, D>(f, n, iters, &matrix)) {
+      if (const int per = swarm_per_block<F, D>(f, n, iters, st, &matrix)) {
         // the slots lie in the workspace: 2 x (32 + 8 D) bytes a block of
         // at least 1024 / D particles, within the positions' and velocities'
         // 16 D n bytes

@@ -27,6 +27,9 @@ namespace zb {
   void set_error(const char* fmt, ...);
   int cuda_fail(cudaError_t e, const char* what);
   int sm_count();
+  // SMs that kernels launched on `st` may use: the device's, or those of the
+  // part of it that the stream's green context or the current context has.
+  int stream_sm_count(cudaStream_t st);
   // The error of a call whose swarm came back with NaN as gbest's value: a
   // block's wait ran out (zb_pso_swarm.cuh).
   int swarm_gave_up();
@@ -45,7 +48,7 @@ namespace zb {
   // for tests that make it run out.
   extern "C" int* zeus_internal_swarm_wait(void);
   // whether launch_pso runs a swarm of n in one launch
-  bool pso_one_launch(const Objective& o, int64_t n, int iters);
+  bool pso_one_launch(const Objective& o, int64_t n, int iters, cudaStream_t st);
   int launch_pso(const Objective& o, uint64_t seed, int64_t n, double lower,
                  double upper, int iters, double w, double c1, double c2,
                  double* pbx, double* pbf, double* gbest, void* ws,

@@ -8,9 +8,11 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include <cooperative_groups.h>
+#include <cuda.h>
 
 #include "zb_internal.h"
 #include "zb_objective_visit.cuh"
@@ -40,6 +42,52 @@ namespace zb {
       return ZEUS_OK;
     set_error("%s: %s", what, cudaGetErrorString(e));
     return e == cudaErrorMemoryAllocation ? ZEUS_E_NOMEM : ZEUS_E_CUDA;
+  }
+
+  int
+  stream_sm_count(cudaStream_t st)
+  {
+    struct Driver {
+      decltype(&cuStreamGetGreenCtx) green = nullptr;
+      decltype(&cuGreenCtxGetDevResource) green_sms = nullptr;
+      decltype(&cuCtxGetCurrent) current = nullptr;
+      decltype(&cuCtxGetDevResource) sms = nullptr;
+      Driver()
+      {
+        const auto get = [](const char* name, auto& fn) {
+          cudaDriverEntryPointQueryResult q;
+          void* p = nullptr;
+          if (cudaGetDriverEntryPointByVersion(name, &p, 12040, cudaEnableDefault, &q) ==
+                cudaSuccess &&
+              q == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<std::remove_reference_t<decltype(fn)>>(p);
+          else
+            cudaGetLastError();
+        };
+        get("cuStreamGetGreenCtx", green);
+        get("cuGreenCtxGetDevResource", green_sms);
+        get("cuCtxGetCurrent", current);
+        get("cuCtxGetDevResource", sms);
+      }
+    };
+    static const Driver d;
+    int n = sm_count();
+    const auto least = [&](CUresult r, const CUdevResource& res) {
+      if (r == CUDA_SUCCESS && (int)res.sm.smCount > 0 && (int)res.sm.smCount < n)
+        n = (int)res.sm.smCount;
+    };
+    CUdevResource res{};
+    CUgreenCtx g = nullptr;
+    // (the default streams have the current context)
+    if (d.green && d.green_sms && st && st != cudaStreamLegacy && st != cudaStreamPerThread &&
+        d.green(st, &g) == CUDA_SUCCESS && g) {
+      least(d.green_sms(g, &res, CU_DEV_RESOURCE_TYPE_SM), res);
+      return n;
+    }
+    CUcontext ctx = nullptr;
+    if (d.current && d.sms && d.current(&ctx) == CUDA_SUCCESS && ctx)
+      least(d.sms(ctx, &res, CU_DEV_RESOURCE_TYPE_SM), res);
+    return n;
   }
 
   int
@@ -609,7 +657,7 @@ zeus_pso_device_prng(const zeus_problem* problem, uint64_t seed, int32_t prng,
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (st)
     cudaStreamIsCapturing(st, &cs);
-  if (!st || cs != cudaStreamCaptureStatusNone || pso_one_launch(o, n, iters))
+  if (!st || cs != cudaStreamCaptureStatusNone || pso_one_launch(o, n, iters, st))
     return launch_pso(o, seed, n, lower, upper, iters, w, c1, c2, d_pbest_x,
                       d_pbest_f, d_gbest, d_workspace, workspace_bytes, st,
                       sobol);
