@@ -118,9 +118,8 @@ namespace zb {
   }
 
   namespace {
-    // Particles a block of the one-launch PSO takes and whether C goes to
-    // shared memory; per = 0: the swarm does not fit, and each iteration is a
-    // launch.  A block holds at least kSwarmElems (particle, coordinate)
+    // Particles a block of the one-launch PSO takes; 0: the swarm does not fit,
+    // and each iteration is a launch.  A block holds at least kSwarmElems (particle, coordinate)
     // elements, so a small swarm is one block and needs no meeting, and a
     // large one is spread over the SMs.
     constexpr int64_t kSwarmElems = 1024;
@@ -131,16 +130,13 @@ namespace zb {
     // for the slowest evaluation (some 10 ms) are then far from their limit,
     // and a launch an iteration is nothing beside longer ones
     constexpr int kSwarmMaxBins = 8192;
-    // what a block's static arrays leave of an SM's shared memory
-    constexpr size_t kSwarmSmem = 227 * 1024 - 1280;
 
     template <class F, int D>
     int
-    swarm_per_block(const F& f, int64_t n, int iters, cudaStream_t st, bool* matrix)
+    swarm_per_block(const F& f, int64_t n, int iters, cudaStream_t st)
     {
       constexpr int64_t limit = kSwarmSmem / sizeof(double);
-      *matrix = false;
-      if (iters < 1)
+      if (!swarm_built<F, D>() || iters < 1)
         return 0; // nothing to meet for
       if constexpr (F::kind == ZEUS_OBJ_POISSON_NLL)
         if (f.nbins > kSwarmMaxBins)
@@ -158,23 +154,20 @@ namespace zb {
         // eight particles and C to a block: with C in L2 the blocks of a
         // launch an iteration hide its latency better, several to an SM
         // (4096 particles at D = 150: 213 us that way, 234 this way)
-        if (per > kPsoDmmaParticles || (int64_t)swarm_doubles<F, D>(per, true) > limit)
+        if (per > kPsoDmmaParticles)
           return 0;
-        *matrix = true;
-      } else if constexpr (F::kind == ZEUS_OBJ_GAUSSIAN) {
-        *matrix = true; // D x D is small
       }
-      if (per > swarm_threads<F, D>() || (int64_t)swarm_doubles<F, D>(per, *matrix) > limit)
+      if (per > swarm_threads<F, D>() || (int64_t)swarm_doubles<F, D>(per) > limit)
         return 0;
       return (int)per;
     }
 
-    template <class F, int D, bool Matrix>
+    template <class F, int D>
     int
     launch_swarm(const F& f, const SwarmArgs& a, unsigned blocks, cudaStream_t st)
     {
-      auto kern = pso_swarm_kernel<F, D, Matrix>;
-      const size_t smem = sizeof(double) * swarm_doubles<F, D>(a.per_block, Matrix);
+      auto kern = pso_swarm_kernel<F, D>;
+      const size_t smem = sizeof(double) * swarm_doubles<F, D>(a.per_block);
       int rc = ZEUS_OK;
       // the most a swarm takes, not what this one takes: the attribute is the
       // kernel's, and a smaller swarm on another thread would lower it between
@@ -221,8 +214,7 @@ namespace zb {
   {
     return visit_objective(o, [&](auto f) -> int {
              using F = decltype(f);
-             bool m;
-             return swarm_per_block<F, (int)F::arity>(f, n, iters, st, &m) > 0 ? 1 : 0;
+             return swarm_per_block<F, (int)F::arity>(f, n, iters, st) > 0 ? 1 : 0;
            }) == 1;
   }
 
@@ -256,22 +248,20 @@ namespace zb {
     return visit_objective(o, [&](auto f) -> int {
       using F = decltype(f);
       constexpr int D = (int)F::arity;
-      bool matrix = false;
-      if (const int per = swarm_per_block<F, D>(f, n, iters, st, &matrix)) {
-        // the slots lie in the workspace: 2 x (32 + 8 D) bytes a block of
-        // at least 1024 / D particles, within the positions' and velocities'
-        // 16 D n bytes
-        const unsigned nb = (unsigned)((n + per - 1) / per);
-        SwarmArgs a{n,     per, iters, lower, upper, w, c1, c2, seed, sobol, pbx, pbf, gbest,
-                    static_cast<unsigned long long*>(ws), nullptr,
-                    *zeus_internal_swarm_wait()};
-        a.slot_x = reinterpret_cast<double*>(a.slots + 8 * (size_t)nb);
-        // (the Gaussian's matrix is always in shared memory)
-        const int rc =
-          launch_swarm<F, D, F::kind == ZEUS_OBJ_GAUSSIAN>(f, a, nb, st);
-        if (rc != kSwarmNoRoom)
-          return rc;
-      }
+      if constexpr (swarm_built<F, D>())
+        if (const int per = swarm_per_block<F, D>(f, n, iters, st)) {
+          // the slots lie in the workspace: 2 x (32 + 8 D) bytes a block of
+          // at least 1024 / D particles, within the positions' and velocities'
+          // 16 D n bytes
+          const unsigned nb = (unsigned)((n + per - 1) / per);
+          SwarmArgs a{n,     per, iters, lower, upper, w, c1, c2, seed, sobol, pbx, pbf, gbest,
+                      static_cast<unsigned long long*>(ws), nullptr,
+                      *zeus_internal_swarm_wait()};
+          a.slot_x = reinterpret_cast<double*>(a.slots + 8 * (size_t)nb);
+          const int rc = launch_swarm<F, D>(f, a, nb, st);
+          if (rc != kSwarmNoRoom)
+            return rc;
+        }
       pso_reset_kernel<D><<<1, 256, 0, st>>>(wk);
       if constexpr (D >= kPsoCoopMinDim && D <= kPsoDmmaMaxDim &&
                     F::kind == ZEUS_OBJ_GAUSSIAN) {

@@ -170,15 +170,29 @@ namespace zb {
 
   // Doubles of shared memory of a block of `per` particles: positions,
   // velocities, bests, terms, values and best values, gbest's position, warp
-  // scratch, flags; and C where `matrix`.
+  // scratch, flags; and the Gaussian's C.
   template <class F, int D>
   constexpr size_t
-  swarm_doubles(int64_t per, bool matrix)
+  swarm_doubles(int64_t per)
   {
     const size_t sd = swarm_stride<F, D>();
     return (size_t)per * (sd + 2 * D + (swarm_terms<F, D>() ? sd : 0) + 2) + D +
            swarm_threads<F, D>() + (size_t)(per + 1) / 2 + 2 +
-           (matrix ? D * (swarm_dmma<F, D>() ? sd : (size_t)D) : 0);
+           (F::kind == 3 ? D * (swarm_dmma<F, D>() ? sd : (size_t)D) : 0);
+  }
+
+  // What a block's static arrays leave of an SM's shared memory.
+  inline constexpr size_t kSwarmSmem = 227 * 1024 - 1280;
+
+  // Whether any swarm of the objective fits a block: a particle, or the eight
+  // of the tensor-core product (D = 150; the kernel's tiles and hand-over
+  // array are laid out for the dimensions that fit, and no others are built).
+  template <class F, int D>
+  constexpr bool
+  swarm_built()
+  {
+    return sizeof(double) * swarm_doubles<F, D>(swarm_dmma<F, D>() ? kPsoDmmaParticles : 1) <=
+           kSwarmSmem;
   }
 
   // f of eight particles (rows of Xs) with C in shared memory, the bits of
@@ -192,6 +206,7 @@ namespace zb {
   {
     constexpr int JT = (D + 7) / 8, KT = (D + 3) / 4;
     static_assert(JT <= NT / 32, "a warp a tile");
+    static_assert((JT - 8) * 64 <= NT, "ex holds the tiles past the eighth");
     const int lane = threadIdx.x & 31, jt = threadIdx.x >> 5;
     const int r = lane >> 2, c4 = lane & 3;
     const double* xr = Xs + r * SD;
@@ -282,16 +297,17 @@ namespace zb {
     key = ((unsigned long long)mh << 32) | ml;
   }
 
-  template <class F, int D, bool Matrix>
+  template <class F, int D>
   __global__ void __launch_bounds__(swarm_threads<F, D>(), 1)
     pso_swarm_kernel(F f, const __grid_constant__ SwarmArgs a)
   {
     constexpr int NT = swarm_threads<F, D>(), SD = swarm_stride<F, D>();
     extern __shared__ __align__(16) double sm[];
     const int per = a.per_block;
-    double* Cs = sm; // C where Matrix
+    constexpr bool kMatrix = F::kind == 3;
+    double* Cs = sm; // C where kMatrix
     constexpr int CS = swarm_dmma<F, D>() ? SD : D; // row stride of C
-    double* X = Cs + (Matrix ? D * CS : 0);
+    double* X = Cs + (kMatrix ? D * CS : 0);
     double* V = X + (size_t)per * SD;
     double* P = V + (size_t)per * D;
     double* T = P + (size_t)per * D;
@@ -314,7 +330,7 @@ namespace zb {
     const int kwarps = (cnt + 31) / 32; // warps that hold a particle's key
     double gbf = __longlong_as_double(0x7ff0000000000000ll);
 
-    if constexpr (Matrix)
+    if constexpr (kMatrix)
 #pragma unroll 10
       for (int e = t; e < D * D; e += NT)
         Cs[e / D * CS + e % D] = f.C[e];
@@ -374,13 +390,12 @@ namespace zb {
         // ahead of the chain of additions
         if (t < cnt) {
           const double* x = X + t * SD;
-          const double* M = Matrix ? Cs : f.C;
           double q = 0.0;
           for (int i = 0; i < D; ++i) {
             const double xi = x[i];
 #pragma unroll(D < 16 ? D : 16)
             for (int j = 0; j < D; ++j)
-              q += xi * M[i * D + j] * x[j];
+              q += xi * Cs[i * D + j] * x[j];
           }
           FV[t] = 0.5 * q;
         }
