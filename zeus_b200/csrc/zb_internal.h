@@ -78,6 +78,10 @@ namespace zb {
 
   // fast-mode layouts (zb_fast_thread.cu, zb_fast_tile.cu, zb_fast_cta.cu)
   bool thread_layout_supported(int kind, int dim);
+  // whether the thread layout gives each of n runs a warp (zb_fast_thread.cu)
+  bool thread_layout_warps(int kind, int dim, int gradient, int max_iter, int64_t n);
+  extern "C" int zeus_internal_thread_layout_warps(int kind, int dim, int gradient,
+                                                   int max_iter, int64_t n);
   int launch_thread(const Objective& o, const zeus_bfgs_config& c,
                     const BfgsParams& prm, const double* starts,
                     const RunOut& out, Control* ctl, cudaStream_t st);
