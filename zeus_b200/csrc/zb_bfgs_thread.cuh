@@ -68,13 +68,30 @@ namespace zb {
     }
   }
 
+  // Whether a thread of the standalone kernel takes ||g|| = sqrt(g.g) only where
+  // it decides something (far above tol^2, g.g cannot pass the test), as a warp
+  // does, and a thread of the batch kernel (the mixed batch 16.1 against 16.6 ms
+  // with a root an iteration).  Here the branch costs more than the root
+  // (8192 Ackley-10 runs 484 us with the root, 517 with the branch; 4096
+  // likelihood fits with dual gradients 60.6 and 65.2 ms; Rosenbrock-4 95
+  // registers and 104), but for the likelihood's adjoint (16384 fits of 300
+  // iterations 74 and 56 ms).
+  template <class F, bool Adjoint>
+  constexpr bool
+  root_rarely()
+  {
+    if constexpr (requires { F::kind; })
+      return Adjoint && F::kind == 4;
+    return false;
+  }
+
   // One run, start x0[D], results to slot idx of `out`, on the calling thread
   // alone (G = 1) or on its warp (G = 32).  On a warp every lane holds the
   // whole run -- x, g, p, H and each scalar, the same bits in all of them --
   // and they differ only in the line search: lane l evaluates trial l, a
   // ballot picks the first that passes.  The values are those of the
   // one-thread form bit for bit, trial by trial and sum by sum.
-  template <class F, int D, bool Adjoint, bool kTimed = false, int G = 1>
+  template <class F, int D, bool Adjoint, bool kTimed = false, int G = 1, bool Rarely = true>
   __device__ __forceinline__ void
   thread_run(const F& f, const BfgsParams& prm, const double* __restrict__ x0,
              int64_t idx, const RunOut& out, Control* ctl)
@@ -217,15 +234,14 @@ namespace zb {
 #pragma unroll
       for (int i = 0; i < D; ++i)
         gg = fma(g[i], g[i], gg);
-      // ||g|| = sqrt(g.g): taken only where it decides something (far
-      // above tol^2, g.g cannot pass the test)
-      if (!isfinite(gg) || !isfinite(fnew)) {
+      const double size = Rarely ? gg : sqrt(gg);
+      if (!isfinite(size) || !isfinite(fnew)) {
         status = kNonFinite;
         fout = fnew;
         gout = sqrt(gg);
         break;
       }
-      if (gg <= tol_sq4 && sqrt(gg) < prm.tol) {
+      if (Rarely ? gg <= tol_sq4 && sqrt(gg) < prm.tol : size < prm.tol) {
         if (lane == 0)
           note_converged(ctl, prm.required);
         status = kConverged;
@@ -286,7 +302,8 @@ namespace zb {
   {
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx < prm.n)
-      thread_run<F, D, Adjoint, kTimed>(f, prm, starts + idx * D, idx, out, ctl);
+      thread_run<F, D, Adjoint, kTimed, 1, root_rarely<F, Adjoint>()>(f, prm, starts + idx * D,
+                                                                      idx, out, ctl);
   }
 
   // A run to a warp.  A launch lasts as long as its slowest runs, those

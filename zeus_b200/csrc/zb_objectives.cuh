@@ -80,12 +80,14 @@ namespace zeus {
     }
 
     // (unrolled whole where a thread holds x in registers: a partly unrolled
-    // loop indexes x dynamically, which puts it in local memory)
+    // loop indexes x dynamically, which puts it in local memory.  Three terms
+    // are whole at 4 too, and scheduled better: D = 4, a thread a run, 32768
+    // runs of 1000 iterations 1.88 against 2.20 ms)
     __host__ __device__ double
     value(const double* x) const
     {
       double sum = 0.0;
-#pragma unroll(D <= 16 ? 16 : 4)
+#pragma unroll(D > 4 && D <= 16 ? 16 : 4)
       for (std::size_t i = 0; i + 1 < D; ++i) {
         const double t1 = 1.0 - x[i];
         const double t2 = fma(-x[i], x[i], x[i + 1]);
