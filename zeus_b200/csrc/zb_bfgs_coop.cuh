@@ -161,7 +161,10 @@ namespace zb {
     constexpr int R = (D + TS - 1) / TS;
     constexpr bool kLine = HasValueLine<F>;
     constexpr bool kCoopFirst = !kLine || D > 8;
-    constexpr bool kSweep = !kLine && has_value_trials<F, TS>();
+    // (not beside a dual gradient, whose iterations are that gradient: the
+    // sweeps' registers halve the warps in flight, 5000 fits of 100 iterations
+    // 66 -> 108 ms)
+    constexpr bool kSweep = !kLine && Adjoint && has_value_trials<F, TS>();
     const int lane = (int)tile.thread_rank();
     double* xs = buf;
     double* gs = xs + D;
@@ -499,10 +502,10 @@ namespace zb {
     grp.sync();
   }
 
-  template <class F, int D, int TS, bool Adjoint, bool kTimed = false>
-  __global__ void __launch_bounds__(kTileBlock)
-    bfgs_tile_kernel(F f, BfgsParams prm, const double* __restrict__ starts,
-                     RunOut out, Control* ctl)
+  template <class F, int D, int TS, bool Adjoint, bool kTimed>
+  __device__ __forceinline__ void
+  tile_block(const F& f, const BfgsParams& prm, const double* __restrict__ starts,
+             const RunOut& out, Control* ctl)
   {
     constexpr int TPB = kTileBlock / TS;
     extern __shared__ __align__(16) double sm[];
@@ -513,6 +516,27 @@ namespace zb {
       return; // the whole tile leaves together
     tile_run<F, D, TS, Adjoint, kTimed>(f, tile, sm + tslot * tile_smem_doubles<D, TS>(),
                                         prm, starts + run * D, run, out, ctl);
+  }
+
+  template <class F, int D, int TS, bool Adjoint, bool kTimed = false>
+  __global__ void __launch_bounds__(kTileBlock)
+    bfgs_tile_kernel(F f, BfgsParams prm, const double* __restrict__ starts,
+                     RunOut out, Control* ctl)
+  {
+    tile_block<F, D, TS, Adjoint, kTimed>(f, prm, starts, out, ctl);
+  }
+
+  // For an objective with value_trials and more runs than the SMs hold at once:
+  // the sweeps of several trials take 217 registers, two blocks to an SM; here
+  // they spill to 96 and five.  A run alone is slower for it (100 bins, 200
+  // iterations: 2.0 against 1.4 ms), a bulk of runs faster (32768 runs of 100
+  // iterations 8.0 against 11.1 ms; without sweeps, 96 registers, 8.2).
+  template <class F, int D, int TS>
+  __global__ void __launch_bounds__(kTileBlock, 5)
+    bfgs_tile_bulk_kernel(F f, BfgsParams prm, const double* __restrict__ starts,
+                          RunOut out, Control* ctl)
+  {
+    tile_block<F, D, TS, true, false>(f, prm, starts, out, ctl);
   }
 
   // ---------------------------------------------------------------- CTA

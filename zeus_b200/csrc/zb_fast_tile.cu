@@ -5,6 +5,18 @@
 namespace zb {
 
   namespace {
+    // Runs from which the sweeps' bulk kernel is the faster one.  One wave of the
+    // other is 1184 runs; above a few of them the time is the bulk's, unless
+    // runs that iterate to MAX_ITER outlast it: they take their time from one
+    // run's iteration.  The lines cross at 4096 runs for 20 to 100 iterations
+    // (4096: 1.90 ms either way at 100), near 5000 for 500, 9000 for 2000, and at
+    // 10000 near 30000 (16384: 124 against 139 ms; 32768: 169 against 171).
+    bool
+    tile_bulk(const BfgsParams& prm)
+    {
+      return prm.n > 4096 + 2 * (int64_t)prm.max_iter;
+    }
+
     template <class F, int D, int TS>
     int
     launch_ts(const F& f, bool adjoint, const BfgsParams& prm,
@@ -16,6 +28,12 @@ namespace zb {
       const size_t smem = sizeof(double) * TPB * tile_smem_doubles<D, TS>();
       // the cycle timers are compiled in only where they are asked for
       const bool timed = out.cycles != nullptr;
+      if constexpr (has_value_trials<F, TS>() && !HasValueLine<F>)
+        if (adjoint && !timed && tile_bulk(prm)) {
+          bfgs_tile_bulk_kernel<F, D, TS>
+            <<<grid, kTileBlock, smem, st>>>(f, prm, starts, out, ctl);
+          return cuda_fail(cudaGetLastError(), "tile-layout BFGS launch");
+        }
       if (adjoint && timed)
         bfgs_tile_kernel<F, D, TS, true, true>
           <<<grid, kTileBlock, smem, st>>>(f, prm, starts, out, ctl);
