@@ -205,9 +205,9 @@ namespace zb {
       grp.template sum<1>(v);
       ddir = v[0];
     }
-    // the stop flag, tested every kStopEvery iterations on the value read at
-    // the previous test
-    int stop = load_stop(ctl);
+    // the stop flag: read every kStopEvery iterations and tested at the next,
+    // which hides its round trip
+    int stop = load_stop(ctl), limit = prm.max_iter;
     const double tol_sq4 = 4.0 * prm.tol * prm.tol;
     bool pend = false;
     bool stalled = false; // the last search ended without a passing trial
@@ -215,13 +215,17 @@ namespace zb {
     int status = kUnset, iter, executed = -1;
     double fout = best, gout = 0.0;
 
-    for (iter = 0; iter < prm.max_iter; ++iter) {
-      if (iter % kStopEvery == 0) {
-        stop = grp.bcast(stop, 0);
-        if (stop) {
+    if (limit > 0 && grp.bcast(stop, 0)) {
+      status = kStopped;
+      limit = 0;
+    }
+    for (iter = 0; iter < limit; ++iter) {
+      if (iter % kStopEvery == 1) {
+        if (grp.bcast(stop, 0)) {
           status = kStopped;
           break;
         }
+      } else if (iter % kStopEvery == 0) {
         stop = load_stop(ctl);
       }
       // ---- line search: alpha_k = 2^-k, first k in 0..19 that passes,
