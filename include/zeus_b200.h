@@ -374,7 +374,11 @@ int zeus_nll_sensitivity_device(const zeus_problem* problem,
  * long as its slowest run, one that iterates to max_iter).  Records the
  * layout with the lowest estimate in a per-process table keyed by (device,
  * kind, dim, gradient); ZEUS_LAYOUT_AUTO launches and batches then use it.
- * Synchronous.  *best_ms is the winner's estimate. */
+ * The thread layout is timed with a thread a run, which batches and launches
+ * of many runs have, and with a warp a run, which launches of few have, and
+ * a choice is recorded for each.  *best_layout, *best_tile and *best_ms (the
+ * winner's estimate) are the choice for a launch like the sample, which is
+ * also what zeus_autotune_lookup gives.  Synchronous. */
 int zeus_autotune(const zeus_problem* problem, const zeus_bfgs_config* config,
                   int64_t n_sample, uint64_t seed, double lower, double upper,
                   int32_t* best_layout, int32_t* best_tile, float* best_ms,
@@ -383,7 +387,8 @@ int zeus_autotune(const zeus_problem* problem, const zeus_bfgs_config* config,
  * the current device, else 0. */
 int zeus_autotune_lookup(int32_t kind, int32_t dim, int32_t gradient,
                          int32_t* layout, int32_t* tile);
-/* Records a choice (e.g. from a previous process) for the current device. */
+/* Records a choice (e.g. from a previous process) for the current device, for
+ * launches of few and of many runs and batches alike. */
 int zeus_autotune_record(int32_t kind, int32_t dim, int32_t gradient,
                          int32_t layout, int32_t tile);
 

@@ -48,7 +48,7 @@ namespace zb {
     {
       *tile = 0;
       int l = 0, t = 0;
-      if (zeus_autotune_lookup(kind, dim, gradient, &l, &t) &&
+      if (autotune_lookup(false, kind, dim, gradient, &l, &t) &&
           batch_layout_ok(kind, dim, l, t)) {
         *layout = l;
         *tile = t;

@@ -60,9 +60,13 @@ namespace zb {
     if (prm.n <= 0)
       return ZEUS_OK;
     int layout = c.layout, tile = c.tile;
-    if (layout == ZEUS_LAYOUT_AUTO &&
-        !zeus_autotune_lookup(o.kind, o.dim, c.gradient, &layout, &tile))
-      default_layout(o.kind, o.dim, &layout, &tile);
+    if (layout == ZEUS_LAYOUT_AUTO) {
+      // what the thread layout would run here is what it was timed with
+      const bool warps = c.block <= 0 && !out.cycles &&
+                         thread_layout_warps(o.kind, o.dim, c.gradient, c.max_iter, prm.n);
+      if (!autotune_lookup(warps, o.kind, o.dim, c.gradient, &layout, &tile))
+        default_layout(o.kind, o.dim, &layout, &tile);
+    }
     switch (layout) {
       case ZEUS_LAYOUT_THREAD:
         if (!thread_layout_supported(o.kind, o.dim))

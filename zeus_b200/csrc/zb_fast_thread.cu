@@ -123,7 +123,8 @@ namespace zb {
         const bool timed = out.cycles != nullptr;
         // (a block size asked for names the thread form)
         if constexpr (!QuadraticForm<F>)
-          if (!timed && c.block <= 0 && warp_per_run<F>(adjoint, prm.max_iter, prm.n))
+          if (!timed && (c.block == kBlockWarps ||
+                         (c.block <= 0 && warp_per_run<F>(adjoint, prm.max_iter, prm.n))))
             return adjoint ? launch_warp<F, D, true>(f, prm, starts, out, ctl, st)
                            : launch_warp<F, D, false>(f, prm, starts, out, ctl, st);
         if (adjoint && timed)

@@ -78,7 +78,10 @@ namespace zb {
 
   // fast-mode layouts (zb_fast_thread.cu, zb_fast_tile.cu, zb_fast_cta.cu)
   bool thread_layout_supported(int kind, int dim);
-  // whether the thread layout gives each of n runs a warp (zb_fast_thread.cu)
+  // zeus_bfgs_config::block for a warp a run at any n (the autotuner's)
+  inline constexpr int kBlockWarps = -0x7fffffff;
+  // whether the thread layout gives each of n runs a warp (zb_fast_thread.cu);
+  // for one run it does wherever it has that form
   bool thread_layout_warps(int kind, int dim, int gradient, int max_iter, int64_t n);
   extern "C" int zeus_internal_thread_layout_warps(int kind, int dim, int gradient,
                                                    int max_iter, int64_t n);
@@ -105,6 +108,9 @@ namespace zb {
   // workspace of a CTA- or row-layout launch: the run queue, and past about
   // D = 160 the CTA blocks' H slices
   size_t cta_workspace_bytes(int dim, int64_t n);
+  // the autotuner's record for standalone launches whose thread layout has a
+  // warp a run, or for the others and batches
+  int autotune_lookup(bool warps, int kind, int dim, int gradient, int* layout, int* tile);
   // default layout / tile width for (kind, dim): ZEUS_LAYOUT_* and width
   void default_layout(int kind, int dim, int* layout, int* tile);
 

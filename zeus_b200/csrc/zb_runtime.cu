@@ -478,10 +478,13 @@ namespace zb {
                                         : fast_workspace_bytes(o, *c, n);
     }
 
-    // Autotuned layouts: (device, kind, dim, gradient) -> (layout, tile).
+    // Autotuned layouts: (device, kind, dim, gradient) -> (layout, tile), for
+    // batches and for launches whose thread layout has a thread a run (0), for
+    // launches whose thread layout has a warp a run (1), and the one of them
+    // that was reported (2).
     struct TuneTable {
       std::mutex mu;
-      std::map<std::tuple<int, int, int, int>, std::pair<int, int>> m;
+      std::map<std::tuple<int, int, int, int>, std::pair<int, int>> m[3];
     };
     TuneTable&
     tune_table()
@@ -529,6 +532,39 @@ namespace zb {
                        "allocation");
     }
 
+    int
+    tune_lookup(int form, int kind, int dim, int gradient, int32_t* layout, int32_t* tile)
+    {
+      int dev = 0;
+      if (cudaGetDevice(&dev) != cudaSuccess)
+        return 0;
+      TuneTable& t = tune_table();
+      std::lock_guard<std::mutex> lk(t.mu);
+      auto it = t.m[form].find(std::make_tuple(dev, kind, dim, gradient));
+      if (it == t.m[form].end())
+        return 0;
+      if (layout)
+        *layout = it->second.first;
+      if (tile)
+        *tile = it->second.second;
+      return 1;
+    }
+
+    int
+    tune_record(int form, int kind, int dim, int gradient, int layout, int tile)
+    {
+      if (layout < ZEUS_LAYOUT_THREAD || layout > ZEUS_LAYOUT_ROWS) {
+        set_error("zeus_autotune_record: layout must be THREAD, TILE, CTA or ROWS");
+        return ZEUS_E_INVALID;
+      }
+      int dev = 0;
+      cudaGetDevice(&dev);
+      TuneTable& t = tune_table();
+      std::lock_guard<std::mutex> lk(t.mu);
+      t.m[form][std::make_tuple(dev, kind, dim, gradient)] = {layout, tile};
+      return ZEUS_OK;
+    }
+
     // Cached executable graphs for the PSO loop, keyed by the launch shape;
     // new pointer arguments go in through cudaGraphExecUpdate.
     struct GraphCache {
@@ -543,6 +579,12 @@ namespace zb {
     }
 
   } // namespace
+
+  int
+  autotune_lookup(bool warps, int kind, int dim, int gradient, int* layout, int* tile)
+  {
+    return tune_lookup(warps ? 1 : 0, kind, dim, gradient, layout, tile);
+  }
 } // namespace zb
 
 using namespace zb;
@@ -1052,34 +1094,16 @@ int
 zeus_autotune_lookup(int32_t kind, int32_t dim, int32_t gradient,
                      int32_t* layout, int32_t* tile)
 {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess)
-    return 0;
-  TuneTable& t = tune_table();
-  std::lock_guard<std::mutex> lk(t.mu);
-  auto it = t.m.find(std::make_tuple(dev, (int)kind, (int)dim, (int)gradient));
-  if (it == t.m.end())
-    return 0;
-  if (layout)
-    *layout = it->second.first;
-  if (tile)
-    *tile = it->second.second;
-  return 1;
+  return tune_lookup(2, kind, dim, gradient, layout, tile);
 }
 
 int
 zeus_autotune_record(int32_t kind, int32_t dim, int32_t gradient,
                      int32_t layout, int32_t tile)
 {
-  if (layout < ZEUS_LAYOUT_THREAD || layout > ZEUS_LAYOUT_ROWS) {
-    set_error("zeus_autotune_record: layout must be THREAD, TILE, CTA or ROWS");
-    return ZEUS_E_INVALID;
-  }
-  int dev = 0;
-  cudaGetDevice(&dev);
-  TuneTable& t = tune_table();
-  std::lock_guard<std::mutex> lk(t.mu);
-  t.m[std::make_tuple(dev, (int)kind, (int)dim, (int)gradient)] = {layout, tile};
+  for (int form = 0; form < 3; ++form)
+    if (int rc = tune_record(form, kind, dim, gradient, layout, tile))
+      return rc;
   return ZEUS_OK;
 }
 
@@ -1102,17 +1126,24 @@ zeus_autotune(const zeus_problem* problem, const zeus_bfgs_config* config,
     return ZEUS_E_INVALID;
   }
   const int kind = problem->kind, dim = problem->dim;
-  std::vector<std::pair<int, int>> cand;
-  if (thread_layout_supported(kind, dim))
-    cand.push_back({ZEUS_LAYOUT_THREAD, 0});
+  // layout, tile, block: the thread layout in either form it may have
+  struct Candidate {
+    int layout, tile, block;
+  };
+  std::vector<Candidate> cand;
+  if (thread_layout_supported(kind, dim)) {
+    cand.push_back({ZEUS_LAYOUT_THREAD, 0, config->block > 0 ? config->block : 128});
+    if (thread_layout_warps(kind, dim, config->gradient, config->max_iter, 1))
+      cand.push_back({ZEUS_LAYOUT_THREAD, 0, kBlockWarps});
+  }
   const unsigned w = tile_widths(kind, dim);
   for (int k = 1; k <= 5; ++k)
     if ((w >> k) & 1u)
-      cand.push_back({ZEUS_LAYOUT_TILE, 1 << k});
+      cand.push_back({ZEUS_LAYOUT_TILE, 1 << k, config->block});
   if (cta_layout_supported(kind, dim))
-    cand.push_back({ZEUS_LAYOUT_CTA, 0});
+    cand.push_back({ZEUS_LAYOUT_CTA, 0, config->block});
   if (rows_layout_supported(kind, dim))
-    cand.push_back({ZEUS_LAYOUT_ROWS, 0});
+    cand.push_back({ZEUS_LAYOUT_ROWS, 0, config->block});
   if (cand.empty()) {
     set_error("zeus_autotune: no layout built for kind %d dim %d", kind, dim);
     return ZEUS_E_UNSUPPORTED;
@@ -1160,16 +1191,15 @@ zeus_autotune(const zeus_problem* problem, const zeus_bfgs_config* config,
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  float best = 3.4e38f;
-  int bl = -1, bt = 0;
-  for (auto [layout, tile] : cand) {
+  // the records' bests: with a thread a run in the thread layout (launches of
+  // many runs, and batches) and with a warp a run
+  float best[2] = {3.4e38f, 3.4e38f};
+  int bl[2] = {-1, -1}, bt[2] = {0, 0};
+  for (const Candidate& cd : cand) {
     zeus_bfgs_config c = *config;
-    c.layout = layout;
-    c.tile = tile;
-    // the record also serves batches, whose kernel runs the thread layout a
-    // thread per run: that form is the one timed
-    if (layout == ZEUS_LAYOUT_THREAD && c.block <= 0)
-      c.block = 128;
+    c.layout = cd.layout;
+    c.tile = cd.tile;
+    c.block = cd.block;
     float ms_min = 3.4e38f;
     for (int rep = 0; rep < 2 && rc == ZEUS_OK; ++rep) { // warm-up + timed
       cudaMemsetAsync(ctl, 0, sizeof(int32_t) * 2, st);
@@ -1215,24 +1245,34 @@ zeus_autotune(const zeus_problem* problem, const zeus_bfgs_config* config,
     // the class alone would take about the longer of its bulk (the sample)
     // and one run iterating to max_iter
     const float est = std::max(ms_min, lat_ms * (float)config->max_iter);
-    if (est < best) {
-      best = est;
-      bl = layout;
-      bt = tile;
-    }
+    const bool thread = cd.layout == ZEUS_LAYOUT_THREAD, warps = cd.block == kBlockWarps;
+    for (int form = 0; form < 2; ++form)
+      if ((!thread || warps == (form == 1)) && est < best[form]) {
+        best[form] = est;
+        bl[form] = cd.layout;
+        bt[form] = cd.tile;
+      }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cleanup();
   if (rc != ZEUS_OK)
     return rc;
-  zeus_autotune_record(kind, dim, config->gradient, bl, bt);
+  for (int form = 0; form < 2; ++form)
+    if (bl[form] > 0)
+      tune_record(form, kind, dim, config->gradient, bl[form], bt[form]);
+  // reported: the choice for a launch like the sample
+  const int rep = config->block <= 0 && thread_layout_warps(kind, dim, config->gradient,
+                                                            config->max_iter, n_sample)
+                    ? 1
+                    : 0;
+  tune_record(2, kind, dim, config->gradient, bl[rep], bt[rep]);
   if (best_layout)
-    *best_layout = bl;
+    *best_layout = bl[rep];
   if (best_tile)
-    *best_tile = bt;
+    *best_tile = bt[rep];
   if (best_ms)
-    *best_ms = best;
+    *best_ms = best[rep];
   return ZEUS_OK;
 }
 
