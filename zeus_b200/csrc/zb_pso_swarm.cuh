@@ -22,9 +22,9 @@
 // The launch is cooperative (every block resident), so the wait is as long as
 // the slowest block's evaluation.  It has a limit all the same: a block that has
 // read the slots SwarmArgs::wait times gives up, fills its rows of pbx and pbf
-// and gbest's value with NaN and returns.  The blocks that wait for it do the
-// same, block 0 among them, so gbest's value is NaN (which no swarm's best is)
-// whenever a row is not the swarm's.
+// with NaN and publishes nothing more.  So block 0, which waits for all in every
+// iteration, gives up as well, and gbest's value is NaN (which no swarm's best
+// is) whenever a row is not the swarm's.
 #pragma once
 
 #include "zb_objectives.cuh"
@@ -542,16 +542,8 @@ namespace zb {
         }
       }
       __syncthreads();
-      if (sh_late) {
-        const double nan = __longlong_as_double(0x7ff8000000000000ll);
-        if (t == 0)
-          a.gbest[0] = nan;
-        for (int e = t; e < elems; e += NT)
-          a.pbx[i0 * D + e] = nan;
-        for (int p = t; p < cnt; p += NT)
-          a.pbf[i0 + p] = nan;
-        return;
-      }
+      if (sh_late)
+        break;
       if (sh_win >= 0 && sh_f < gbf) {
         gbf = sh_f;
         const int win = sh_win;
@@ -586,13 +578,15 @@ namespace zb {
       }
     }
     __syncthreads();
+    const bool late = sh_late != 0;
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
     for (int e = t; e < elems; e += NT)
-      a.pbx[i0 * D + e] = P[e];
+      a.pbx[i0 * D + e] = late ? nan : P[e];
     for (int p = t; p < cnt; p += NT)
-      a.pbf[i0 + p] = PF[p];
+      a.pbf[i0 + p] = late ? nan : PF[p];
     if (blockIdx.x == 0) {
       if (t == 0)
-        a.gbest[0] = gbf;
+        a.gbest[0] = late ? nan : gbf;
       for (int d = t; d < D; d += NT)
         a.gbest[1 + d] = gb[d];
     }
