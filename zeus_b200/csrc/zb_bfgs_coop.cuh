@@ -206,8 +206,10 @@ namespace zb {
       ddir = v[0];
     }
     // the stop flag: read every kStopEvery iterations and tested at the next,
-    // which hides its round trip
-    int stop = load_stop(ctl), limit = prm.max_iter;
+    // which hides its round trip.  (A first test ahead of the loop, and a
+    // read in the test's else, made the compiler spend other registers on the
+    // loop: 5000 Ackley-10 runs 245 -> 279 us, Rastrigin-16 5% slower.)
+    int stop = load_stop(ctl);
     const double tol_sq4 = 4.0 * prm.tol * prm.tol;
     bool pend = false;
     bool stalled = false; // the last search ended without a passing trial
@@ -215,19 +217,16 @@ namespace zb {
     int status = kUnset, iter, executed = -1;
     double fout = best, gout = 0.0;
 
-    if (limit > 0 && grp.bcast(stop, 0)) {
-      status = kStopped;
-      limit = 0;
-    }
-    for (iter = 0; iter < limit; ++iter) {
-      if (iter % kStopEvery == 1) {
-        if (grp.bcast(stop, 0)) {
+    for (iter = 0; iter < prm.max_iter; ++iter) {
+      if (iter % kStopEvery == 1 || iter == 0) {
+        stop = grp.bcast(stop, 0);
+        if (stop) {
           status = kStopped;
           break;
         }
-      } else if (iter % kStopEvery == 0) {
-        stop = load_stop(ctl);
       }
+      if (iter % kStopEvery == 0)
+        stop = load_stop(ctl);
       // ---- line search: alpha_k = 2^-k, first k in 0..19 that passes,
       // else alpha = 2^-20 (utils.cuh:376-412)
       int found = -1;
