@@ -111,8 +111,8 @@ def algorithmic_flops(jobs_counters) -> float:
 #  * gaussian150: the quadratic-form BFGS kernel at full size (C, the starts
 #    and the first touch of the outputs).
 MEASURED_TRAFFIC = {
-    "mixed": (8 * (600064 + 1024), "1/8-size capture x 8, batch kernel"),
-    "gaussian150": (1466000, "full-size capture"),
+    "mixed": (8 * 504064, "1/8-size capture x 8, batch kernel"),
+    "gaussian150": (1467136 + 3584, "full-size capture"),
 }
 
 

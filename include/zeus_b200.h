@@ -254,6 +254,10 @@ int zeus_pso_device_noalloc(const zeus_problem* problem, uint64_t seed,
  * line search, update skip, accept-if-better and termination protocol.
  * d_control: 2 int32 {stop flag, converged count}, zeroed by the caller
  * before the first launch (the reference's BFGSContext, context.hpp:7-10).
+ * The run that makes the required count raises the flag; the others end with
+ * status 2 one to five iterations later (five to eight where the thread
+ * layout has a warp a run), and those that converge in between count as
+ * converged.  A flag that is up before a launch ends every run at its start.
  * Workspace: zeus_bfgs_workspace_size() bytes: none for the thread and tile
  * layouts; the CTA layout (dim > 32) keeps its blocks' run queue there (a
  * block that finishes a run takes the next unstarted one) and, past about

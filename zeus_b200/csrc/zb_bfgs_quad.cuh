@@ -17,8 +17,8 @@
 // column pair's rows q, q + Q, ... -- so H lives in its registers but for
 // KS rows, and C takes H's place in shared memory, copied once per block for
 // all the runs it takes.  An iteration at D = 150 is then 7500 cycles: 2400 the
-// pass over C (2100 shared-memory wavefronts), 2000 the sweep (six FP64
-// operations an element), 3100 the partial sums, two reductions and the O(D)
+// pass over C (2100 shared-memory wavefronts), 1600 the sweep (six FP64
+// operations an element), 3500 the partial sums, two reductions and the O(D)
 // work, a chain of latencies.  1024 runs 1106 -> 673 us on a B200, 64 runs
 // 723 -> 439, 8192 runs 5280 -> 3167.  A run on a cluster of two blocks, each
 // with half the columns, was shorter alone (64 runs: 377 us) but two blocks'

@@ -310,13 +310,14 @@ namespace zb {
   // that iterate to MAX_ITER: there no trial passes, and one thread
   // evaluates 21 of them one after another while its warp's other lanes
   // wait.  All 21 at once leave the chain of one evaluation, one gradient
-  // and the update, 0.36 us an iteration at D = 2 against 1.05 and 0.85
-  // against 4.0 at D = 8 (B200, 1965 MHz; a good part of the latter is the
-  // objective's unrolling, see Rosenbrock::adjoint).  1024 Rosenbrock-2 runs
-  // 10.5 -> 3.9 ms, 4096 Rosenbrock-8 runs 41.7 -> 8.8, 16384 Rastrigin-2 runs
-  // 54 -> 6.4, 16384 Ackley-2 runs 72 -> 14; widths of 16 and 8 lanes measured
-  // slower throughout (10.0 and 12.4 ms for 16384 Rosenbrock-2 runs, 8.1 on
-  // 32).
+  // and the update, 0.35 us an iteration at D = 2 against 1.04 and 0.59
+  // against 3.7 at D = 8, one run alone (B200, 1965 MHz; a good part of the
+  // latter is the objective's unrolling, see Rosenbrock::adjoint).  1024
+  // Rosenbrock-2 runs 10.5 -> 3.9 ms, 4099 Rosenbrock-8 runs 40.2 -> 8.8 or
+  // 12.9 (by which SM partitions the 44 that iterate to MAX_ITER share), 16384
+  // Rastrigin-2 runs 54 -> 6.4, 16384 Ackley-2 runs 72 -> 14; widths of 16 and 8
+  // lanes measured slower throughout (10.0 and 12.4 ms for 16384 Rosenbrock-2
+  // runs, 8.1 on 32).
   inline constexpr int kThreadGroupBlock = 64;
 
   template <class F, int D, bool Adjoint>

@@ -164,8 +164,12 @@ namespace zb {
   // Relaxed read of the stop flag (the reference's atomicAdd(&stopFlag, 0),
   // once an iteration, bfgs_common.cuh:127).  Its round trip to L2 is as long as
   // a short iteration, and a barrier waits for the loads its threads have in
-  // flight, so a group reads it every kStopEvery iterations and sees a raised
-  // flag that much later.
+  // flight, so the tile layout, a warp of the thread layout and the
+  // quadratic-form kernel read it every kStopEvery iterations.  A run there sees
+  // a raised flag two to five iterations later (tile), five to eight (warp,
+  // which tests the value read four before: a test one iteration after the read
+  // was within an iteration's length of the round trip and cost 2-4%) or within
+  // four (quadratic form); elsewhere within one to three.
   inline constexpr int kStopEvery = 4;
   __device__ __forceinline__ int
   load_stop(const Control* c)

@@ -4,10 +4,11 @@
 // positions, velocities and bests that go out to memory and back, and on a
 // last block that reduces while the others wait: 14 us an iteration for 16384
 // particles at D = 10 and for 1024 at D = 150, where the arithmetic is 1-2 us.
-// One launch: 16384 Rastrigin-10 particles, 20 iterations, 315 -> 126 us; 1024
-// Gaussian-150 particles, 10 iterations, 204 -> 126 us, 4700 of an iteration's
-// cycles the tensor-core product and 3000 the meeting; 20000 Rosenbrock-32
-// particles, 10 iterations, 485 -> 113 us (B200).
+// One launch: 16384 Rastrigin-10 particles, 20 iterations, 291 -> 94 us; 1024
+// Gaussian-150 particles, 10 iterations, 159 -> 71 us (of a 77 us build's
+// iteration 5500 cycles were the tensor-core product, 2960 of them its issue,
+// and 3000 the meeting); 20000 Rosenbrock-32 particles, 10 iterations, 487 -> 104
+// us (B200).
 // Here a block keeps its particles' state in shared memory for the whole
 // call.  Its threads take (particle, coordinate) elements, so the random
 // numbers and moves of one particle are spread over D threads; where the
