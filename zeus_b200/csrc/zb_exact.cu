@@ -123,9 +123,6 @@ namespace zb {
     // elements, so a small swarm is one block and needs no meeting, and a
     // large one is spread over the SMs.
     constexpr int64_t kSwarmElems = 1024;
-    // the driver has no room for all blocks at once after all: each iteration
-    // is a launch
-    constexpr int kSwarmNoRoom = 1;
     // bins up to which a likelihood's swarm is one launch: the blocks that wait
     // for the slowest evaluation (some 10 ms) are then far from their limit,
     // and a launch an iteration is nothing beside longer ones
@@ -195,8 +192,8 @@ namespace zb {
       lc.numAttrs = blocks > 1 ? 1 : 0;
       const cudaError_t e = cudaLaunchKernelEx(&lc, kern, f, a);
       if (e == cudaErrorCooperativeLaunchTooLarge) {
-        cudaGetLastError();
-        return kSwarmNoRoom;
+        cudaGetLastError(); // no room for all blocks at once after all
+        return kPsoNotOne;
       }
       return cuda_fail(e, "PSO launch");
     }
@@ -209,20 +206,11 @@ namespace zb {
     return &wait;
   }
 
-  bool
-  pso_one_launch(const Objective& o, int64_t n, int iters, cudaStream_t st)
-  {
-    return visit_objective(o, [&](auto f) -> int {
-             using F = decltype(f);
-             return swarm_per_block<F, (int)F::arity>(f, n, iters, st) > 0 ? 1 : 0;
-           }) == 1;
-  }
-
   int
   launch_pso(const Objective& o, uint64_t seed, int64_t n, double lower,
              double upper, int iters, double w, double c1, double c2,
              double* pbx, double* pbf, double* gbest, void* ws,
-             size_t ws_bytes, cudaStream_t st, const uint32_t* sobol)
+             size_t ws_bytes, cudaStream_t st, const uint32_t* sobol, PsoPath path)
   {
     if (n <= 0)
       return ZEUS_OK;
@@ -249,7 +237,8 @@ namespace zb {
       using F = decltype(f);
       constexpr int D = (int)F::arity;
       if constexpr (swarm_built<F, D>())
-        if (const int per = swarm_per_block<F, D>(f, n, iters, st)) {
+        if (const int per = path == PsoPath::steps ? 0
+                                                   : swarm_per_block<F, D>(f, n, iters, st)) {
           // the slots lie in the workspace: 2 x (32 + 8 D) bytes a block of
           // at least 1024 / D particles, within the positions' and velocities'
           // 16 D n bytes
@@ -259,9 +248,11 @@ namespace zb {
                       *zeus_internal_swarm_wait()};
           a.slot_x = reinterpret_cast<double*>(a.slots + 8 * (size_t)nb);
           const int rc = launch_swarm<F, D>(f, a, nb, st);
-          if (rc != kSwarmNoRoom)
+          if (rc != kPsoNotOne)
             return rc;
         }
+      if (path == PsoPath::one)
+        return kPsoNotOne;
       pso_reset_kernel<D><<<1, 256, 0, st>>>(wk);
       if constexpr (D >= kPsoCoopMinDim && D <= kPsoDmmaMaxDim &&
                     F::kind == ZEUS_OBJ_GAUSSIAN) {

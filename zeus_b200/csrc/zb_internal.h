@@ -47,13 +47,15 @@ namespace zb {
   // The calling thread's limit on the one-launch PSO's wait (SwarmArgs::wait),
   // for tests that make it run out.
   extern "C" int* zeus_internal_swarm_wait(void);
-  // whether launch_pso runs a swarm of n in one launch
-  bool pso_one_launch(const Objective& o, int64_t n, int iters, cudaStream_t st);
+  // which of launch_pso's paths: one launch where the swarm fits, else a launch
+  // an iteration; the first alone (kPsoNotOne where it does not fit); the second
+  enum class PsoPath { any, one, steps };
+  inline constexpr int kPsoNotOne = 1;
   int launch_pso(const Objective& o, uint64_t seed, int64_t n, double lower,
                  double upper, int iters, double w, double c1, double c2,
                  double* pbx, double* pbf, double* gbest, void* ws,
                  size_t ws_bytes, cudaStream_t st,
-                 const uint32_t* sobol = nullptr);
+                 const uint32_t* sobol = nullptr, PsoPath path = PsoPath::any);
 
   // Tile widths built for an objective and dimension (bit k: width 2^k):
   // H rows per lane R*D <= 64 doubles; up to 4*D lanes (the spare lanes

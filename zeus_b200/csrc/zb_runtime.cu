@@ -699,10 +699,12 @@ zeus_pso_device_prng(const zeus_problem* problem, uint64_t seed, int32_t prng,
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (st)
     cudaStreamIsCapturing(st, &cs);
-  if (!st || cs != cudaStreamCaptureStatusNone || pso_one_launch(o, n, iters, st))
-    return launch_pso(o, seed, n, lower, upper, iters, w, c1, c2, d_pbest_x,
-                      d_pbest_f, d_gbest, d_workspace, workspace_bytes, st,
-                      sobol);
+  const bool direct = !st || cs != cudaStreamCaptureStatusNone;
+  rc = launch_pso(o, seed, n, lower, upper, iters, w, c1, c2, d_pbest_x, d_pbest_f, d_gbest,
+                  d_workspace, workspace_bytes, st, sobol,
+                  direct ? PsoPath::any : PsoPath::one);
+  if (direct || rc != kPsoNotOne)
+    return rc;
   // A launch an iteration: capture them into one graph and launch it.
   rc = cuda_fail(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal),
                  "PSO capture begin");
@@ -710,7 +712,8 @@ zeus_pso_device_prng(const zeus_problem* problem, uint64_t seed, int32_t prng,
     return rc;
   const int lrc =
     launch_pso(o, seed, n, lower, upper, iters, w, c1, c2, d_pbest_x,
-               d_pbest_f, d_gbest, d_workspace, workspace_bytes, st, sobol);
+               d_pbest_f, d_gbest, d_workspace, workspace_bytes, st, sobol,
+               PsoPath::steps);
   cudaGraph_t graph = nullptr;
   const cudaError_t ec = cudaStreamEndCapture(st, &graph);
   if (lrc) {
